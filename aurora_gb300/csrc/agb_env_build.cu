@@ -298,8 +298,7 @@ __global__ void k_env_alias(const double* p, const float* lum, uint32_t n, const
 // The reference's table (AliasMap.cpp:71-166) rebuilt bit for bit: FP32 luminance x row solid
 // angle (row angles from the host, as the reference computes them), FP32 sequential integral, the
 // same index map (below-average texels first in index order, the others from the end), and the
-// same sequential sweep.  The sweep is inherently sequential; one warp runs it, lanes prefetching
-// the next windows of the small and large queues into shared memory while lane 0 consumes them.
+// same sequential sweep.
 
 __global__ void k_ref_lum(const float4* rgba, uint32_t width, uint32_t n, const float* rowSA,
     float* lum, float* lumArea)
@@ -314,30 +313,192 @@ __global__ void k_ref_lum(const float4* rgba, uint32_t width, uint32_t n, const 
     lumArea[i] = __fmul_rn(rowSA[i / width], l);
 }
 
-// One warp: FP32 sum of v[0, n) in index order, as a sequential loop would compute it.
-__global__ void k_ref_seq_sum(const float* v, uint32_t n, float* out)
+// FP32 sum of v[0, n) in index order, bit for bit as a sequential loop computes it, by one block.
+//
+// While the running sum stays in one binade its ulp u is fixed and the sum is an integer m of
+// [2^23, 2^24) ulps, so adding v = (q + f) u (q whole, 0 <= f < 1) rounds to m + q, to m + q + 1, or,
+// at f = 1/2, to the even one of the two: every addend is a map m -> m + a[m & 1], and such maps
+// compose into maps of the same kind.  A block scan over kSumPer addends per thread therefore gives
+// every thread the sum that the sequential loop would reach before its addends; a chunk is taken as a
+// whole while no thread's sum leaves the binade.  The first thread that leaves it (or that holds an
+// addend that is negative or not finite) adds its own addends one by one, and the next chunk starts
+// behind them in the new binade.  A sum that is zero, subnormal, infinite or NaN is carried on one by
+// one, in runs that double while that lasts.
+//
+// Bound by the load and scan latency of one block, a few us per chunk of 8,192 addends and per binade:
+// 512 x 256 texels 0.63 ms by the sequential loop (10 cycles an addend), 0.11 ms so.  Whole-number
+// arithmetic: the same maps from FP64 products took 0.63 ms too (two FP64 lanes' worth per SM).
+constexpr int kSumThreads   = 1024;
+constexpr int kSumPer       = 8;
+constexpr uint32_t kSumFull = 1u << 24; // one past the binade's last integer
+constexpr uint32_t kSumCap  = 1u << 25; // saturation of the maps: any value beyond kSumFull does
+
+struct SumMap
 {
-    constexpr uint32_t kChunk = 4096;
-    __shared__ float buf[kChunk];
-    int lane  = threadIdx.x;
-    float acc = 0.f;
-    for (uint32_t base = 0; base < n; base += kChunk)
+    uint32_t a0, a1; // added to an even / odd integer
+};
+__device__ __forceinline__ SumMap composeSum(SumMap f, SumMap g)
+{
+    SumMap h;
+    h.a0 = min(f.a0 + ((f.a0 & 1u) ? g.a1 : g.a0), kSumCap);
+    h.a1 = min(f.a1 + (((f.a1 + 1u) & 1u) ? g.a1 : g.a0), kSumCap);
+    return h;
+}
+
+__global__ void __launch_bounds__(kSumThreads) k_ref_seq_sum(const float* v, uint32_t n, float* out)
+{
+    __shared__ SumMap warpMap[kSumThreads / 32];
+    __shared__ float accS;
+    __shared__ uint32_t posS;
+    __shared__ int firstStop;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    float acc       = 0.f;
+    uint32_t pos    = 0;
+    uint32_t serial = 64; // addends of the next one-by-one run
+    while (pos < n)
     {
-        uint32_t cnt = n - base < kChunk ? n - base : kChunk;
-        for (uint32_t k = lane; k < cnt; k += 32)
-            buf[k] = v[base + k];
-        __syncwarp();
+        if (!(acc >= 1.17549435e-38f && acc < __int_as_float(0x7f800000)))
+        {
+            if (acc == 0.f)
+            {
+                // Zeros leave a zero sum as it is: on to the first addend that is not one (its group of 8).
+                uint32_t first = uint32_t(kSumThreads * kSumPer);
+#pragma unroll
+                for (int k = kSumPer - 1; k >= 0; k--)
+                {
+                    const uint32_t i = pos + uint32_t(k) * kSumThreads + t;
+                    if (i < n && v[i] != 0.f)
+                        first = uint32_t(k) * kSumThreads + t;
+                }
+                if (t == 0)
+                    posS = kSumThreads * kSumPer;
+                __syncthreads();
+                atomicMin(&posS, first);
+                __syncthreads();
+                pos = min(pos + (posS & ~uint32_t(kSumPer - 1)), n);
+                __syncthreads();
+                if (pos == n)
+                    continue;
+            }
+            const uint32_t cnt = min(serial, n - pos);
+            if (t == 0)
+            {
+                float s = acc;
+                for (uint32_t k = 0; k < cnt; k++)
+                    s = __fadd_rn(s, v[pos + k]);
+                accS = s;
+            }
+            __syncthreads();
+            acc = accS;
+            pos += cnt;
+            serial = min(serial * 2u, 8192u);
+            __syncthreads();
+            continue;
+        }
+        serial = 64;
+        const int e        = int(__float_as_uint(acc) >> 23); // biased exponent, 1 .. 254
+        const uint32_t m0  = (__float_as_uint(acc) & 0x7fffffu) | 0x800000u;
+        const uint32_t at  = pos + uint32_t(t) * kSumPer;
+        float x[kSumPer];
+        if (at + kSumPer <= n)
+        {
+            const float4 p = *reinterpret_cast<const float4*>(v + at), q = *reinterpret_cast<const float4*>(v + at + 4);
+            x[0] = p.x, x[1] = p.y, x[2] = p.z, x[3] = p.w;
+            x[4] = q.x, x[5] = q.y, x[6] = q.z, x[7] = q.w;
+        }
+        else
+#pragma unroll
+            for (int k = 0; k < kSumPer; k++)
+                x[k] = at + k < n ? v[at + k] : 0.f;
+        SumMap mine{ 0u, 0u };
+        bool odd = false; // an addend that the maps do not describe
+#pragma unroll
+        for (int k = 0; k < kSumPer; k++)
+        {
+            odd             = odd || !(x[k] >= 0.f && x[k] < __int_as_float(0x7f800000));
+            // v = M 2^(ev - 150) (M < 2^24) is M / 2^sh ulps of the sum, sh = e - ev.
+            const uint32_t bits = __float_as_uint(x[k]);
+            const int eb        = int(bits >> 23) & 255;
+            const uint32_t M    = (bits & 0x7fffffu) | (eb ? 0x800000u : 0u);
+            const int sh        = e - (eb ? eb : 1);
+            SumMap g;
+            if (sh > 0)
+            {
+                const int s1        = min(sh, 26); // from 25 on the addend is below half an ulp
+                const uint32_t q    = M >> s1;
+                const uint32_t rem2 = (M & ((1u << s1) - 1u)) << 1, one = 1u << s1; // 2 f against 1
+                g.a0 = q + (rem2 > one ? 1u : (rem2 == one ? (q & 1u) : 0u));
+                g.a1 = q + (rem2 > one ? 1u : (rem2 == one ? ((q + 1u) & 1u) : 0u));
+            }
+            else
+                g.a0 = g.a1 = M == 0u ? 0u : (sh < -2 ? kSumCap : min(M << -sh, kSumCap));
+            mine = composeSum(mine, g);
+        }
+        // Inclusive scan of the maps in thread order, then the map before this thread.
+        SumMap incl = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            SumMap o{ __shfl_up_sync(0xffffffffu, incl.a0, off), __shfl_up_sync(0xffffffffu, incl.a1, off) };
+            if (lane >= off)
+                incl = composeSum(o, incl);
+        }
+        SumMap excl{ __shfl_up_sync(0xffffffffu, incl.a0, 1), __shfl_up_sync(0xffffffffu, incl.a1, 1) };
         if (lane == 0)
-            for (uint32_t k = 0; k < cnt; k++)
-                acc = __fadd_rn(acc, buf[k]);
-        __syncwarp();
+            excl = SumMap{ 0u, 0u };
+        if (lane == 31)
+            warpMap[warp] = incl;
+        if (t == 0)
+            firstStop = kSumThreads;
+        __syncthreads();
+        if (warp == 0)
+        {
+            SumMap w = warpMap[lane];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1)
+            {
+                SumMap o{ __shfl_up_sync(0xffffffffu, w.a0, off), __shfl_up_sync(0xffffffffu, w.a1, off) };
+                if (lane >= off)
+                    w = composeSum(o, w);
+            }
+            SumMap b{ __shfl_up_sync(0xffffffffu, w.a0, 1), __shfl_up_sync(0xffffffffu, w.a1, 1) };
+            if (lane == 0)
+                b = SumMap{ 0u, 0u };
+            warpMap[lane] = b;
+        }
+        __syncthreads();
+        const SumMap before   = composeSum(warpMap[warp], excl);
+        const SumMap after    = composeSum(before, mine);
+        const uint32_t mStart = m0 + ((m0 & 1u) ? before.a1 : before.a0);
+        const uint32_t mEnd   = m0 + ((m0 & 1u) ? after.a1 : after.a0);
+        if ((odd || mEnd >= kSumFull) && mStart < kSumFull)
+            atomicMin(&firstStop, t);
+        __syncthreads();
+        // mStart < kSumFull holds for every thread up to the first one that stops.
+        const int stop = firstStop;
+        if (stop == kSumThreads ? t == kSumThreads - 1 : t == stop)
+        {
+            const uint32_t m = stop == kSumThreads ? mEnd : mStart;
+            float s          = __uint_as_float((uint32_t(e) << 23) | (m & 0x7fffffu));
+            if (stop != kSumThreads)
+#pragma unroll
+                for (int k = 0; k < kSumPer; k++)
+                    if (at + k < n)
+                        s = __fadd_rn(s, x[k]);
+            accS = s;
+            posS = pos + uint32_t(stop == kSumThreads ? kSumThreads : stop + 1) * kSumPer;
+        }
+        __syncthreads();
+        acc = accS;
+        pos = posS;
+        __syncthreads();
     }
-    if (lane == 0)
+    if (t == 0)
         *out = acc;
 }
 
 __global__ void k_ref_probs(const float* lum, const float* lumArea, uint32_t n,
-    const float* integral, float* prob, float* pdf, uint32_t* alias, uint32_t* tileSmall)
+    const float* integral, float* prob, float* pdf, uint32_t* tileSmall)
 {
     uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     float I       = *integral;
@@ -351,7 +512,6 @@ __global__ void k_ref_probs(const float* lum, const float* lumArea, uint32_t n,
         float pr = __fdiv_rn(lumArea[i], average);
         prob[i]  = pr;
         pdf[i]   = __fdiv_rn(lum[i], I);
-        alias[i] = i;
         smalls += pr < 1.f ? 1u : 0u;
     }
     double t;
@@ -360,8 +520,9 @@ __global__ void k_ref_probs(const float* lum, const float* lumArea, uint32_t n,
         tileSmall[blockIdx.x] = uint32_t(t);
 }
 
+// The index map, and in its order the probabilities and (each entry its own) the aliases.
 __global__ void k_ref_index(const float* prob, uint32_t n, const uint32_t* tileSmallExcl,
-    uint32_t* indexMap)
+    uint32_t* indexMap, float* posProb, uint32_t* posAlias)
 {
     uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t smalls = 0;
@@ -379,115 +540,125 @@ __global__ void k_ref_index(const float* prob, uint32_t n, const uint32_t* tileS
         uint32_t i = base + q;
         if (i >= n)
             break;
-        if (isSmall[q])
-            indexMap[before++] = i;
-        else
-            indexMap[n - 1 - (i - before)] = i; // k-th large (index order) at position n-1-k
+        // The k-th large (index order) at position n - 1 - k.
+        const uint32_t pos = isSmall[q] ? before++ : n - 1 - (i - before);
+        indexMap[pos] = i;
+        posProb[pos]  = prob[i];
+        posAlias[pos] = pos;
     }
 }
 
 // The sweep: for (sml = 0; sml < lrg && lrg < n; sml++) pair indexMap[sml] with indexMap[lrg].
-__global__ void k_ref_sweep(const uint32_t* indexMap, float* prob, uint32_t* alias, uint32_t n,
+//
+// The chain w -= 1 - p is sequential (a large's leftover decides where the next one starts), so its
+// latency is the bound: one thread walks it, with everything else taken off its path.  Probabilities
+// and aliases are held in position order, so both queues are plain streams: the block stages a window
+// of each in shared memory (the smalls as their deficits 1 - p, the larges as their p), the walk only
+// subtracts, compares and notes which large a small went to and what a large was left with, and the
+// block writes those notes back.  w never grows within a large (deficits are >= 0), so the walk tests
+// groups of four smalls with one comparison and goes back into a group only when the large ends inside
+// it.  Positions in [S, lrg) are larges already exhausted, whose probability is final and which follow
+// the smalls as smalls; a window beyond S ends at the lrg it started with.
+//
+// 512 x 256 texels of log-normal(0, 2) radiance with four suns: 16.4 ms with one warp that fetched,
+// compared and stored small by small, 2.5 ms so (about 35 cycles a small).
+constexpr int kSweepThreads = 1024;
+constexpr int kSweepWin     = 2048; // window of both queues (a multiple of 4)
+__global__ void __launch_bounds__(kSweepThreads) k_ref_sweep(float* posProb, uint32_t* posAlias, uint32_t n,
     const uint32_t* smallCount)
 {
-    constexpr int kWin = 256; // queue window per batch (8 entries per lane)
-    __shared__ uint32_t sIdx[kWin], lIdx[kWin];
-    __shared__ float sProb[kWin], lProb[kWin];
-    __shared__ uint8_t sFinal[kWin];
-    __shared__ uint32_t st[3]; // sml, lrg, done
-    int lane = threadIdx.x;
-    uint32_t S = *smallCount;
-    uint32_t curLarge = 0;
-    float w = 0.f;
-    if (lane == 0)
+    __shared__ __align__(16) float def[kSweepWin + 4]; // the walk loads one group ahead
+    __shared__ float lrgP[kSweepWin + 3]; // the walk reads up to two larges past the window
+    __shared__ __align__(8) uint16_t owner[kSweepWin]; // large (of the window) that took the small
+    __shared__ uint32_t takenS, endedS;                // smalls consumed, larges ended
+    __shared__ float wS;
+    const int t      = threadIdx.x;
+    const uint32_t S = *smallCount;
+    if (S == 0 || S >= n)
+        return;
+    uint32_t sml = 0, lrg = S;
+    float w = posProb[S]; // of the current large
+    while (sml < lrg && lrg < n)
     {
-        st[0] = 0;
-        st[1] = S;
-        st[2] = (S == 0 || S >= n) ? 1u : 0u;
-        if (!st[2])
+        const uint32_t cntS = min(uint32_t(kSweepWin), (sml < S ? S : lrg) - sml);
+        const uint32_t cntL = min(uint32_t(kSweepWin), n - lrg);
+        for (uint32_t k = t; k < cntS; k += kSweepThreads)
+            def[k] = __fsub_rn(1.f, posProb[sml + k]);
+        for (uint32_t k = t; k < cntL; k += kSweepThreads)
+            lrgP[k] = posProb[lrg + k];
+        if (t < 3)
+            lrgP[cntL + t] = 0.f;
+        __syncthreads();
+        if (t == 0)
         {
-            curLarge = indexMap[S];
-            w        = prob[curLarge];
-        }
-    }
-    __syncwarp();
-    while (!st[2])
-    {
-        uint32_t sml = st[0], lrg = st[1];
-        // Prefetch the small-queue window [sml, sml + kWin) and the large-queue window
-        // (lrg, lrg + kWin].  Small entries below S never change; entries at positions in
-        // [S, lrg) are larges already exhausted, whose probability is final.
-        for (int k = lane; k < kWin; k += 32)
-        {
-            uint32_t ps = sml + uint32_t(k);
-            if (ps < n)
+            uint32_t si = 0, li = 0;
+            float next1 = lrgP[1], next2 = lrgP[2];
+            auto step = [&](float d, uint32_t at) {
+                owner[at]        = uint16_t(li);
+                w                = __fsub_rn(w, d);
+                const bool ended = w < 1.f;
+                if (ended)
+                    lrgP[li] = w;
+                w     = ended ? next1 : w;
+                next1 = ended ? next2 : next1;
+                li += ended ? 1u : 0u;
+                if (ended)
+                    next2 = lrgP[li + 2];
+            };
+            float4 ahead = *reinterpret_cast<const float4*>(def);
+            while (si + 4 <= cntS && li + 4 <= cntL)
             {
-                uint32_t idx = indexMap[ps];
-                sIdx[k]      = idx;
-                bool fin     = ps < S || ps < lrg;
-                sFinal[k]    = fin ? 1 : 0;
-                sProb[k]     = fin ? prob[idx] : 0.f;
-            }
-            uint32_t pl = lrg + 1u + uint32_t(k);
-            if (pl < n)
-            {
-                uint32_t idx = indexMap[pl];
-                lIdx[k]      = idx;
-                lProb[k]     = prob[idx]; // untouched until it becomes the current large
-            }
-        }
-        __syncwarp();
-        if (lane == 0)
-        {
-            int si = 0, li = 0;
-            while (si < kWin && li < kWin)
-            {
-                if (!(sml < lrg && lrg < n))
+                const float4 d = ahead; // the next group is loaded while this one is walked
+                ahead          = *reinterpret_cast<const float4*>(def + si + 4);
+                const float w3 = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(w, d.x), d.y), d.z), d.w);
+                if (!(w3 < 1.f))
                 {
-                    st[2] = 1;
-                    break;
+                    *reinterpret_cast<uint2*>(owner + si) = make_uint2(li | (li << 16), li | (li << 16));
+                    w = w3;
                 }
-                uint32_t small = sIdx[si];
-                float ps       = sFinal[si] ? sProb[si] : prob[small];
-                alias[small]   = curLarge;
-                w              = __fsub_rn(w, __fsub_rn(1.f, ps));
-                if (w < 1.f)
+                else
                 {
-                    prob[curLarge] = w;
-                    lrg++;
-                    if (lrg < n)
-                    {
-                        curLarge = lIdx[li];
-                        w        = lProb[li];
-                        li++;
-                    }
+                    step(d.x, si);
+                    step(d.y, si + 1);
+                    step(d.z, si + 2);
+                    step(d.w, si + 3);
                 }
-                sml++;
+                si += 4;
+            }
+            while (si < cntS && li < cntL)
+            {
+                step(def[si], si);
                 si++;
             }
-            st[0] = sml;
-            st[1] = lrg;
-            if (lrg >= n || sml >= lrg)
-                st[2] = 1;
-            if (st[2] && lrg < n)
-                prob[curLarge] = w;
+            takenS = si;
+            endedS = li;
+            wS     = w;
         }
-        __syncwarp();
+        __syncthreads();
+        const uint32_t taken = takenS, ended = endedS;
+        for (uint32_t k = t; k < taken; k += kSweepThreads)
+            posAlias[sml + k] = lrg + owner[k];
+        for (uint32_t k = t; k < ended; k += kSweepThreads)
+            posProb[lrg + k] = lrgP[k];
+        sml += taken;
+        lrg += ended;
+        // The large that is current next: carried on, or (the window of larges used up) not yet loaded.
+        w = ended < cntL ? wS : (lrg < n ? posProb[lrg] : 0.f);
+        __syncthreads();
     }
+    if (t == 0 && lrg < n)
+        posProb[lrg] = w;
 }
 
-__global__ void k_ref_pack(const uint32_t* alias, const float* prob, const float* pdf, uint32_t n,
-    agb_alias_entry* out)
+__global__ void k_ref_pack(const uint32_t* indexMap, const uint32_t* posAlias, const float* posProb, const float* pdf,
+    uint32_t n, agb_alias_entry* out)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
+    uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos >= n)
         return;
-    agb_alias_entry e;
-    e.alias     = alias[i];
-    e.prob      = prob[i];
-    e.pdf       = pdf[i];
-    e._padding1 = 0.f;
-    out[i]      = e;
+    const uint32_t i = indexMap[pos];
+    reinterpret_cast<float4*>(out)[i] =
+        make_float4(__uint_as_float(indexMap[posAlias[pos]]), posProb[pos], pdf[i], 0.f);
 }
 
 } // namespace
@@ -571,12 +742,13 @@ cudaError_t launchEnvAliasBuild(const float4* rgba, uint32_t width, uint32_t hei
     else
     {
         // Reference layout.  Scratch reuse: lumArea / prob / pdf in the FP64 weight arrays,
-        // alias / index map in the FP64 prefix arrays.
+        // index map, aliases and position-order probabilities in the FP64 prefix arrays.
         float* lumArea    = reinterpret_cast<float*>(s.scanA);
         float* prob       = reinterpret_cast<float*>(s.scanA) + n;
         float* pdf        = reinterpret_cast<float*>(s.heavyIncl);
-        uint32_t* alias   = reinterpret_cast<uint32_t*>(s.heavyIncl) + n;
+        uint32_t* posAlias = reinterpret_cast<uint32_t*>(s.heavyIncl) + n;
         uint32_t* indexMap = reinterpret_cast<uint32_t*>(s.lightIncl);
+        float* posProb     = reinterpret_cast<float*>(s.lightIncl) + n;
         uint32_t* smallCount = lightCount;
         if (rowSolidAngle)
         {
@@ -586,13 +758,13 @@ cudaError_t launchEnvAliasBuild(const float4* rgba, uint32_t width, uint32_t hei
                 return e;
         }
         k_ref_lum<<<(n + 255) / 256, 256, 0, st>>>(rgba, width, n, s.rowSA, lum, lumArea);
-        k_ref_seq_sum<<<1, 32, 0, st>>>(lumArea, n, shadingIntegral);
+        k_ref_seq_sum<<<1, kSumThreads, 0, st>>>(lumArea, n, shadingIntegral);
         k_ref_probs<<<tiles, kScanThreads, 0, st>>>(lum, lumArea, n, shadingIntegral, prob, pdf,
-            alias, s.blockCounts);
+            s.blockCounts);
         k_scan_tiles_u32<<<1, kScanThreads, 0, st>>>(s.blockCounts, tiles, smallCount);
-        k_ref_index<<<tiles, kScanThreads, 0, st>>>(prob, n, s.blockCounts, indexMap);
-        k_ref_sweep<<<1, 32, 0, st>>>(indexMap, prob, alias, n, smallCount);
-        k_ref_pack<<<(n + 255) / 256, 256, 0, st>>>(alias, prob, pdf, n, out);
+        k_ref_index<<<tiles, kScanThreads, 0, st>>>(prob, n, s.blockCounts, indexMap, posProb, posAlias);
+        k_ref_sweep<<<1, kSweepThreads, 0, st>>>(posProb, posAlias, n, smallCount);
+        k_ref_pack<<<(n + 255) / 256, 256, 0, st>>>(indexMap, posAlias, posProb, pdf, n, out);
     }
     cudaError_t e = cudaMemcpyAsync(integralFP64Out, integral, sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess)
