@@ -653,8 +653,9 @@ AGB_API agb_status agb_geometry_create(agb_context* ctx, const float* positions,
             "agb_geometry_create: GPU BVH build");
         if (depth > kBlasMaxDepth)
             return fail(AGB_ERR_LIMIT, "agb_geometry_create: BLAS deeper than the traversal stack allows");
-        // The builder numbers nodes level by level, so the first ones are the top of the tree.
-        std::vector<BNode> top(std::min<uint32_t>(nodeCount, 255));
+        // The builder numbers the large nodes first, level by level, then each small subtree's in one run:
+        // the first ones are the top of the tree (all of a mesh whose top five levels hold subtrees).
+        std::vector<BNode> top(std::min<uint32_t>(nodeCount, 4096));
         if (!top.empty())
             AGB_CUDA(cudaMemcpyAsync(top.data(), s.nodes, top.size() * sizeof(BNode), cudaMemcpyDeviceToHost,
                          ctx->stream),
