@@ -1911,8 +1911,8 @@ AGB_API agb_status agb_batch_render(agb_batch* b, agb_context* const* views, con
         wb.counters       = W->counters.as<uint32_t>();
         DevScene shared   = b->sceneTable[0];
         shared.ground     = DevGroundPlane{};
-        launchBatchWave(shared, frames[0], wp, wb, bt, maxDepth, forceOpaque != 0, W->stream, W->smCount, launches,
-            marks);
+        launchBatchWave(shared, frames[0], wp, wb, bt, maxDepth, forceOpaque != 0, stats != nullptr, W->stream, W->smCount,
+            launches, marks);
         AGB_CUDA(cudaGetLastError(), "launch batch wave");
         if (stats)
         {

@@ -93,10 +93,11 @@ cudaError_t launchVertexRecords(const float* positions, const float* normals, co
 void launchWave(const DevScene& s, const agb_frame_data& f, const WaveParams& wp,
     const WaveBuffers& wb, cudaStream_t st, int smCount, uint64_t& launches, KernelMarks* marks);
 // A batched wave over several requests (BatchTables): `shared` is the scenes' shared namespace,
-// maxDepth the deepest request's trace depth.
+// maxDepth the deepest request's trace depth; stageLaunches: one launch per stage of the wavefront, for
+// callers that report them.
 void launchBatchWave(const DevScene& shared, const agb_frame_data& anyFrame, const WaveParams& wp,
-    const WaveBuffers& wb, const BatchTables& bt, int maxDepth, bool forceOpaque, cudaStream_t st, int smCount,
-    uint64_t& launches, KernelMarks* marks);
+    const WaveBuffers& wb, const BatchTables& bt, int maxDepth, bool forceOpaque, bool stageLaunches, cudaStream_t st,
+    int smCount, uint64_t& launches, KernelMarks* marks);
 void setTraceAttributes();
 
 // agb_env_build.cu: environment sampling table on the device.  rgba: device RGBA32F texels.

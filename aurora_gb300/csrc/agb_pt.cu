@@ -280,11 +280,11 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM) k_trace_closes
     bool overflow   = false;
     QueueRayLoader rays{ wb.rayOrg[cur], wb.rayDir[cur] };
     if constexpr (kBatch)
-        persistentTrace<false, kCount>(s, n, wb.counters + bounce * kCounterStride + CNT_CLOSEST_WORK,
+        persistentTrace<false, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + CNT_CLOSEST_WORK,
             BatchQueueRayLoader{ rays, wb.rayPath[cur], bt.pathReq, bt.req, bounce },
             HitWriter{ wb.hitTUV, wb.hitInst }, g_stack + threadIdx.x, kTraceBlock, c, overflow);
     else
-        persistentTrace<false, kCount>(s, n, wb.counters + bounce * kCounterStride + CNT_CLOSEST_WORK, rays,
+        persistentTrace<false, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + CNT_CLOSEST_WORK, rays,
             HitWriter{ wb.hitTUV, wb.hitInst }, g_stack + threadIdx.x, kTraceBlock, c, overflow);
     if (kCount)
     {
@@ -306,11 +306,11 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM) k_trace_shadow
     bool overflow   = false;
     ShadowLoader rays{ wb.shTag, wb.shOrg, wb.shDir };
     if constexpr (kBatch)
-        persistentTrace<true, kCount>(s, n, wb.counters + bounce * kCounterStride + workSlot,
+        persistentTrace<true, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + workSlot,
             BatchShadowLoader{ rays, bt.pathReq, bt.req }, OcclusionWriter{ wb.shTag, wb.occluded },
             g_stack + threadIdx.x, kTraceBlock, c, overflow);
     else
-        persistentTrace<true, kCount>(s, n, wb.counters + bounce * kCounterStride + workSlot, rays,
+        persistentTrace<true, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + workSlot, rays,
             OcclusionWriter{ wb.shTag, wb.occluded }, g_stack + threadIdx.x, kTraceBlock, c, overflow);
     if (kCount)
     {
@@ -330,18 +330,75 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM) k_trace_shadow
     bool overflow   = false;
     TransparentShadowLoader rays{ ShadowLoader{ wb.shTag, wb.shOrg, wb.shDir }, wb.shadePoint };
     if constexpr (kBatch)
-        persistentTrace<false, kCount>(s, n, wb.counters + bounce * kCounterStride + CNT_SHADOW_WORK,
+        persistentTrace<false, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + CNT_SHADOW_WORK,
             BatchTransparentShadowLoader{ rays, bt.pathReq, bt.req },
             TransparentShadowWriter{ wb.shTag, wb.shadePoint, wb.pendSlot }, g_stack + threadIdx.x,
             kTraceBlock, c, overflow);
     else
-        persistentTrace<false, kCount>(s, n, wb.counters + bounce * kCounterStride + CNT_SHADOW_WORK, rays,
+        persistentTrace<false, kCount>(s, n, spreadLanes(n), wb.counters + bounce * kCounterStride + CNT_SHADOW_WORK, rays,
             TransparentShadowWriter{ wb.shTag, wb.shadePoint, wb.pendSlot }, g_stack + threadIdx.x,
             kTraceBlock, c, overflow);
     if (kCount)
     {
         atomicAdd(statPtr(wb, 5), c.nodes);
         atomicAdd(statPtr(wb, 6), c.tris);
+    }
+    if (overflow)
+        atomicAdd(statPtr(wb, 4), 1ull);
+}
+
+// The closest-hit rays of bounce + 1 (queue `next`), then the shadow rays of `bounce`, in one launch:
+// neither needs the other's results, and warps that are done with the first queue work on the second
+// while slower ones finish, so one launch has one tail of slow rays (100-170 us) where two have two.  A lone
+// 1920x1080 render of 16 samples of the large scene type 65.5 -> 63.2 ms, a 640x360 one of 1 sample 3.09 ->
+// 2.22 ms.  Two copies of the traversal in one kernel keep its 64 registers (12 bytes spilled); one loop
+// over the two, with blocks that start on either, spilled 200 and was slower on full queues.
+template <bool kBatch, bool kTransparent>
+__global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM) k_trace_both(DevScene s, WaveBuffers wb, int bounce,
+    int next, BatchTables bt)
+{
+    TraceCounters c = { 0, 0 };
+    bool overflow   = false;
+    {
+        uint32_t* then   = wb.counters + (bounce + 1) * kCounterStride;
+        const uint32_t n = then[CNT_RAYS];
+        QueueRayLoader rays{ wb.rayOrg[next], wb.rayDir[next] };
+        const HitWriter hits{ wb.hitTUV, wb.hitInst };
+        if constexpr (kBatch)
+            persistentTrace<false, false>(s, n, spreadLanes(n), then + CNT_CLOSEST_WORK,
+                BatchQueueRayLoader{ rays, wb.rayPath[next], bt.pathReq, bt.req, bounce + 1 }, hits,
+                g_stack + threadIdx.x, kTraceBlock, c, overflow);
+        else
+            persistentTrace<false, false>(s, n, spreadLanes(n), then + CNT_CLOSEST_WORK, rays, hits,
+                g_stack + threadIdx.x, kTraceBlock, c, overflow);
+    }
+    {
+        uint32_t* here   = wb.counters + bounce * kCounterStride;
+        uint32_t* work   = here + CNT_SHADOW_WORK;
+        const uint32_t n = here[CNT_SHADOW];
+        ShadowLoader rays{ wb.shTag, wb.shOrg, wb.shDir };
+        if constexpr (kTransparent)
+        {
+            const TransparentShadowLoader load{ rays, wb.shadePoint };
+            const TransparentShadowWriter write{ wb.shTag, wb.shadePoint, wb.pendSlot };
+            if constexpr (kBatch)
+                persistentTrace<false, false>(s, n, spreadLanes(n), work,
+                    BatchTransparentShadowLoader{ load, bt.pathReq, bt.req }, write, g_stack + threadIdx.x, kTraceBlock,
+                    c, overflow);
+            else
+                persistentTrace<false, false>(s, n, spreadLanes(n), work, load, write, g_stack + threadIdx.x,
+                    kTraceBlock, c, overflow);
+        }
+        else
+        {
+            const OcclusionWriter write{ wb.shTag, wb.occluded };
+            if constexpr (kBatch)
+                persistentTrace<true, false>(s, n, spreadLanes(n), work, BatchShadowLoader{ rays, bt.pathReq, bt.req },
+                    write, g_stack + threadIdx.x, kTraceBlock, c, overflow);
+            else
+                persistentTrace<true, false>(s, n, spreadLanes(n), work, rays, write, g_stack + threadIdx.x, kTraceBlock,
+                    c, overflow);
+        }
     }
     if (overflow)
         atomicAdd(statPtr(wb, 4), 1ull);
@@ -1502,8 +1559,8 @@ __global__ void k_bin_scatter(WaveParams wp, WaveBuffers wb, int bounce, int src
 // opaque shadows as `forceOpaque` says.
 template <bool kBatch>
 void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& wp, const WaveBuffers& wb,
-    const BatchTables& bt, int depth, bool forceOpaque, cudaStream_t st, int smCount, uint64_t& launches,
-    KernelMarks* marks)
+    const BatchTables& bt, int depth, bool forceOpaque, bool stageLaunches, cudaStream_t st, int smCount,
+    uint64_t& launches, KernelMarks* marks)
 {
     auto mark = [&](int category) {
         if (marks)
@@ -1517,6 +1574,7 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
     launches++;
     int cur = 0;
     size_t stackBytes = kTraceStackBytes;
+    const bool apart  = stageLaunches || marks || wp.countTraversal;
     for (int b = 0; b <= depth; b++)
     {
         if (b == depth)
@@ -1529,11 +1587,18 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
             launches++;
             break;
         }
-        mark(KC_CLOSEST);
-        if (wp.countTraversal)
-            k_trace_closest<true, kBatch><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, cur, bt);
-        else
-            k_trace_closest<false, kBatch><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, cur, bt);
+        // The first bounce's closest-hit rays, and every bounce's when the traversals are counted, the launches
+        // timed by family or a batch's statistics asked for (one launch per stage); otherwise they were
+        // traced with the last bounce's shadow rays.
+        if (b == 0 || apart)
+        {
+            mark(KC_CLOSEST);
+            if (wp.countTraversal)
+                k_trace_closest<true, kBatch><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, cur, bt);
+            else
+                k_trace_closest<false, kBatch><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, cur, bt);
+            launches++;
+        }
         if (!kBatch && s.ground.enabled)
         {
             // Ground plane for the bounce's primary rays before they are shaded.
@@ -1559,8 +1624,27 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
         k_shade_scatter<kBatch><<<shadeGrid, kShadeBlock, 0, st>>>(s, f, wp, wb, b, cur, bt);
         mark(KC_SHADE);
         k_shade_mis<kBatch><<<shadeGrid, kShadeBlock, 0, st>>>(s, f, wp, wb, b, bt);
+        int next = cur ^ 1; // queue of the next bounce's rays
+        if (!kBatch && wp.binRays && b + 1 < depth)
+        {
+            // The next bounce's rays, binned from queue cur ^ 1 back into queue cur (free since
+            // this bounce's shading).
+            mark(KC_RESOLVE);
+            k_bin_count<<<grid, 256, 0, st>>>(wp, wb, b + 1, next);
+            k_bin_scan<<<1, 1024, 0, st>>>(wb);
+            k_bin_scatter<<<grid, 256, 0, st>>>(wp, wb, b + 1, next);
+            launches += 3;
+            next = cur;
+        }
         mark(KC_SHADOW);
-        if (!forceOpaque)
+        if (!apart && b + 1 < depth)
+        {
+            if (!forceOpaque)
+                k_trace_both<kBatch, true><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, next, bt);
+            else
+                k_trace_both<kBatch, false><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, next, bt);
+        }
+        else if (!forceOpaque)
         {
             if (wp.countTraversal)
                 k_trace_shadow_transparent<true, kBatch><<<traceGrid, kTraceBlock, stackBytes, st>>>(s, wb, b, bt);
@@ -1575,19 +1659,8 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
                 CNT_SHADOW_WORK, bt);
         mark(KC_RESOLVE);
         k_resolve<kBatch><<<grid, 256, 0, st>>>(f, wb, b, bt);
-        launches += 6;
-        if (!kBatch && wp.binRays && b + 1 < depth)
-        {
-            // The next bounce's rays, binned from queue cur ^ 1 back into queue cur (free since
-            // this bounce's shading).
-            mark(KC_RESOLVE);
-            k_bin_count<<<grid, 256, 0, st>>>(wp, wb, b + 1, cur ^ 1);
-            k_bin_scan<<<1, 1024, 0, st>>>(wb);
-            k_bin_scatter<<<grid, 256, 0, st>>>(wp, wb, b + 1, cur ^ 1);
-            launches += 3;
-        }
-        else
-            cur ^= 1;
+        launches += 5;
+        cur = next;
     }
     mark(KC_FINALIZE);
 #if AGB_SAMPLE_INNER
@@ -1626,15 +1699,15 @@ void launchWave(const DevScene& s, const agb_frame_data& f, const WaveParams& wp
     const WaveBuffers& wb, cudaStream_t st, int smCount, uint64_t& launches, KernelMarks* marks)
 {
     BatchTables none{};
-    launchWaveT<false>(s, f, wp, wb, none, f.trace_depth, f.is_force_opaque_shadows_enabled != 0, st, smCount,
-        launches, marks);
+    launchWaveT<false>(s, f, wp, wb, none, f.trace_depth, f.is_force_opaque_shadows_enabled != 0, false, st,
+        smCount, launches, marks);
 }
 
 void launchBatchWave(const DevScene& shared, const agb_frame_data& anyFrame, const WaveParams& wp,
-    const WaveBuffers& wb, const BatchTables& bt, int maxDepth, bool forceOpaque, cudaStream_t st, int smCount,
-    uint64_t& launches, KernelMarks* marks)
+    const WaveBuffers& wb, const BatchTables& bt, int maxDepth, bool forceOpaque, bool stageLaunches, cudaStream_t st,
+    int smCount, uint64_t& launches, KernelMarks* marks)
 {
-    launchWaveT<true>(shared, anyFrame, wp, wb, bt, maxDepth, forceOpaque, st, smCount, launches, marks);
+    launchWaveT<true>(shared, anyFrame, wp, wb, bt, maxDepth, forceOpaque, stageLaunches, st, smCount, launches, marks);
 }
 
 template <class K>
@@ -1656,6 +1729,10 @@ void setTraceAttributes()
     traceAttributes(k_trace_shadow<false, false>, stackBytes, carveout);
     traceAttributes(k_trace_shadow<true, true>, stackBytes, carveout);
     traceAttributes(k_trace_shadow<false, true>, stackBytes, carveout);
+    traceAttributes(k_trace_both<false, false>, stackBytes, carveout);
+    traceAttributes(k_trace_both<false, true>, stackBytes, carveout);
+    traceAttributes(k_trace_both<true, false>, stackBytes, carveout);
+    traceAttributes(k_trace_both<true, true>, stackBytes, carveout);
     traceAttributes(k_trace_shadow_transparent<true, false>, stackBytes, carveout);
     traceAttributes(k_trace_shadow_transparent<false, false>, stackBytes, carveout);
     traceAttributes(k_trace_shadow_transparent<true, true>, stackBytes, carveout);

@@ -296,8 +296,22 @@ AGB_D int32_t rayRoot(const Loader& load, const DevScene& s, uint32_t i)
         return s.instanceCount > 0 ? s.tlasRoot : kDone;
 }
 
+// Lanes of a warp that take rays from a queue of n: all 32, except that a queue of at most two rays per
+// resident warp is spread over all of them.  The lanes of a warp run their node, leaf and boundary phases
+// for one another, so a ray among 32 divergent ones takes about 1,200 ns per node visit however idle the
+// chip is, and the slowest ray sets the launch's time.  Device time of a lone 640x360 one-sample render
+// of the large scene type 2.22 ms with full warps and 1.89 ms so, of a 160x120 preview 0.90 and 0.77 ms.
+// Spreading larger queues makes that 1.87 ms at most and costs throughput where other streams could use
+// the idle warps (that render beside two others: 0.95 ms with full warps, 0.92 so, 1.13 with every queue
+// spread).
+AGB_D uint32_t spreadLanes(uint32_t n)
+{
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return n <= warps ? 1u : n <= 2u * warps ? 2u : 32u;
+}
+
 template <bool kAnyHit, bool kCount, class Loader, class Writer>
-AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t* work, const Loader& load,
+AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32_t* work, const Loader& load,
     const Writer& write, int32_t* stack, int stride, TraceCounters& cnt, bool& overflow)
 {
     constexpr int kParkLeaves    = kAnyHit ? kParkLeavesAny : kParkLeavesClosest;
@@ -305,7 +319,7 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t* work, const 
     static_assert(kParkLeaves == 1 || kParkLeaves == 2, "one or two parked leaves");
     const unsigned FULL = 0xffffffffu;
     const int lane      = threadIdx.x & 31;
-    bool active = false, exhausted = false;
+    bool active = false, exhausted = uint32_t(lane) >= lanes;
     uint32_t rayIdx = 0;
     v3 o = splat(0.f), d = splat(0.f);
     float tmin = 0.f, tmax = 0.f, tmaxRay = 0.f;

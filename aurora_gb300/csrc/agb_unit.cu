@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_intersect_batch(DevScene s, con
 {
     TraceCounters c = { 0, 0 };
     bool overflow   = false;
-    persistentTrace<kAnyHit, false>(s, n, work, BatchRayLoader{ rays }, BatchHitWriter{ outTUV, outIP },
+    persistentTrace<kAnyHit, false>(s, n, spreadLanes(n), work, BatchRayLoader{ rays }, BatchHitWriter{ outTUV, outIP },
         u_stack + threadIdx.x, kTraceBlock, c, overflow);
     if (overflow)
         atomicAdd(overflowCount, 1ull);
