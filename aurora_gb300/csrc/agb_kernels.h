@@ -24,14 +24,17 @@ inline int traceCarveoutPercent()
     size_t pct  = (need * 100 + 228 * 1024 - 1) / (228 * 1024);
     return int(pct > 100 ? 100 : pct);
 }
-constexpr int kShadeBlock       = 128;
-#ifndef AGB_SHADE_MIN_BLOCKS
-#define AGB_SHADE_MIN_BLOCKS 16
-#endif
-// Resident shading blocks per SM the register budget is sized for.  The shading kernel waits on
-// scattered loads (vertices, materials, textures, environment); full occupancy hides more of that
-// latency than the registers it gives up (measured: 16 blocks of 128 threads beat 8 by 1.3x).
-constexpr int kShadeMinBlocks   = AGB_SHADE_MIN_BLOCKS;
+// Threads per block of the shading kernels, and the resident blocks their register budgets are sized for.
+// They wait on scattered loads (vertices, materials, textures, environment) and on instruction fetch, and at
+// 32 registers (64 warps per SM) they also spilled 1 KB (surface) and 0.3 KB (BSDF kernels) per thread, whose
+// traffic cost more than the occupancy gave: surface kernel 1.85 ms at 32 registers, 1.49 at 40, 1.10 at 64,
+// 0.93 at 128; sampling kernel 1.55, 1.64, 1.33 and 1.65; MIS kernel 1.14, 1.08, 0.91 and 1.13 (512x512x16
+// of the small scene type).  Large blocks keep the warps that share an instruction cache near one another
+// in the code: the sampling kernel at 64 registers 1.33 ms with 128 threads per block, 1.22 with 512.
+constexpr int kShadeBlock     = 256; // surface kernel
+constexpr int kShadeMinBlocks = 2;
+constexpr int kBsdfBlock      = 512; // sampling and MIS kernels
+constexpr int kBsdfMinBlocks  = 2;
 
 // Kernel categories for per-kernel device timing.
 enum KernelCategory

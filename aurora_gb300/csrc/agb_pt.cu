@@ -806,7 +806,7 @@ AGB_D void storeMis(float4* mp, uint32_t stride, uint32_t j, v3 L, float pdf, v3
 }
 
 template <bool kBatch>
-__global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade_scatter(DevScene s,
+__global__ void __launch_bounds__(kBsdfBlock, kBsdfMinBlocks) k_shade_scatter(DevScene s,
     agb_frame_data f, WaveParams wp, WaveBuffers wb, int bounce, int cur, BatchTables bt)
 {
     uint32_t n      = wb.counters[bounce * kCounterStride + CNT_SCATTER];
@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade_scatter(
 }
 
 template <bool kBatch>
-__global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade_mis(DevScene s,
+__global__ void __launch_bounds__(kBsdfBlock, kBsdfMinBlocks) k_shade_mis(DevScene s,
     agb_frame_data f, WaveParams wp, WaveBuffers wb, int bounce, BatchTables bt)
 {
     uint32_t n      = wb.counters[bounce * kCounterStride + CNT_SCATTER];
@@ -1567,7 +1567,7 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
             marks->record(category, st);
     };
     int grid = smCount * 8;
-    int shadeGrid = smCount * (kShadeMinBlocks > 8 ? kShadeMinBlocks : 8);
+    int shadeGrid = smCount * 8, bsdfGrid = smCount * 4;
     int traceGrid = smCount * kTraceBlocksPerSM;
     mark(KC_CAMERA);
     k_camera<kBatch><<<grid, 256, 0, st>>>(f, wp, wb, bt);
@@ -1621,9 +1621,9 @@ void launchWaveT(const DevScene& s, const agb_frame_data& f, const WaveParams& w
         else
             k_shade<kBatch><<<shadeGrid, kShadeBlock, 0, st>>>(s, f, wp, wb, b, cur, 0, bt);
         mark(KC_SHADE);
-        k_shade_scatter<kBatch><<<shadeGrid, kShadeBlock, 0, st>>>(s, f, wp, wb, b, cur, bt);
+        k_shade_scatter<kBatch><<<bsdfGrid, kBsdfBlock, 0, st>>>(s, f, wp, wb, b, cur, bt);
         mark(KC_SHADE);
-        k_shade_mis<kBatch><<<shadeGrid, kShadeBlock, 0, st>>>(s, f, wp, wb, b, bt);
+        k_shade_mis<kBatch><<<bsdfGrid, kBsdfBlock, 0, st>>>(s, f, wp, wb, b, bt);
         int next = cur ^ 1; // queue of the next bounce's rays
         if (!kBatch && wp.binRays && b + 1 < depth)
         {
