@@ -130,7 +130,7 @@ struct agb_context
     DevBuf matGraph, graphOps, graphConsts; // material node-graph programs
     bool hasGraphs = false;
 
-    DevBuf instances, tlasNodes, tlasOrder, layers;
+    DevBuf instances, tlasNodes, tlasOrder, traceInst, layers;
     std::vector<std::unique_ptr<DevBuf>> layerUVs;
     uint32_t instanceCount = 0;
     int32_t tlasRoot       = 0;
@@ -203,7 +203,7 @@ struct agb_context
         s.tlas          = tlasNodes.as<BNode>();
         s.tlasRoot      = tlasRoot;
         s.instanceCount = int32_t(instanceCount);
-        s.tlasOrder     = tlasOrder.as<int32_t>();
+        s.traceInst     = traceInst.as<TraceInstance>();
         s.materials     = materials.as<agb_material>();
         s.matTex        = hasMatTex ? matTex.as<agb_material_textures>() : nullptr;
         s.materialCount = int32_t(materialCount);
@@ -535,7 +535,7 @@ AGB_API agb_status agb_context_memory(agb_context* ctx, uint64_t* bytes)
     if (!ctx || !bytes)
         return fail(AGB_ERR_INVALID_ARG, "agb_context_memory: null argument");
     uint64_t b = ctx->meshTable.bytes + ctx->imageTable.bytes + ctx->materials.bytes +
-        ctx->matTex.bytes + ctx->instances.bytes + ctx->tlasNodes.bytes + ctx->tlasOrder.bytes +
+        ctx->matTex.bytes + ctx->instances.bytes + ctx->tlasNodes.bytes + ctx->tlasOrder.bytes + ctx->traceInst.bytes +
         ctx->layers.bytes + ctx->alias.bytes + ctx->pathState.bytes + ctx->queues.bytes +
         ctx->counters.bytes + ctx->accMean.bytes + ctx->accSum.bytes + ctx->accComp.bytes +
         ctx->lastSample.bytes + ctx->accMoments.bytes + ctx->aovDepth.bytes + ctx->aovNormal.bytes +
@@ -1166,6 +1166,10 @@ AGB_API agb_status agb_instances_set(agb_context* ctx, const agb_instance* inst,
     }
     if (tlasDepth + maxBlas + 2 > kStackSize)
         return fail(AGB_ERR_LIMIT, "agb_instances_set: TLAS + BLAS depth exceeds the traversal stack");
+    AGB_CUDA(ctx->traceInst.ensure(std::max<size_t>(1, count) * sizeof(TraceInstance)), "allocate instance records");
+    AGB_CUDA(launchTraceInstances(ctx->tlasOrder.as<int32_t>(), ctx->instances.as<DevInstance>(),
+                 ctx->meshTable.as<DevMesh>(), count, ctx->traceInst.as<TraceInstance>(), ctx->stream),
+        "build instance records");
     AGB_CUDA(cudaStreamSynchronize(ctx->stream), "upload instances");
     ctx->layerUVs      = std::move(uvs);
     ctx->instanceCount = count;
@@ -1552,7 +1556,7 @@ struct agb_batch
     // Shared namespace of the scenes of the last call.
     std::vector<const agb_context*> scenes;
     std::vector<uint64_t> versions;
-    DevBuf meshes, instances, tlas, tlasOrder, materials, matTex, images, layers;
+    DevBuf meshes, instances, tlas, tlasOrder, traceInst, materials, matTex, images, layers;
     std::vector<DevScene> sceneTable;
     DevBuf sceneTableDev, reqTable, frameTable, pathReq;
     cudaEvent_t done = nullptr;
@@ -1672,12 +1676,16 @@ agb_status buildSharedScenes(agb_batch* b, const std::vector<agb_context*>& scen
         (r = put(b->tlas, N.data(), N.size() * sizeof(BNode), "batch TLAS")) ||
         (r = put(b->tlasOrder, O.data(), O.size() * sizeof(int32_t), "batch TLAS order")))
         return r;
+    AGB_CUDA(b->traceInst.ensure(std::max<size_t>(1, O.size()) * sizeof(TraceInstance)), "batch instance records");
+    AGB_CUDA(launchTraceInstances(b->tlasOrder.as<int32_t>(), b->instances.as<DevInstance>(), b->meshes.as<DevMesh>(),
+                 uint32_t(O.size()), b->traceInst.as<TraceInstance>(), st),
+        "batch instance records");
     for (DevScene& e : table)
     {
         e.meshes        = b->meshes.as<DevMesh>();
         e.instances     = b->instances.as<DevInstance>();
         e.tlas          = b->tlas.as<BNode>();
-        e.tlasOrder     = b->tlasOrder.as<int32_t>();
+        e.traceInst     = b->traceInst.as<TraceInstance>();
         e.materials     = b->materials.as<agb_material>();
         e.matTex        = anyTex ? b->matTex.as<agb_material_textures>() : nullptr;
         e.materialCount = int32_t(Mt.size());

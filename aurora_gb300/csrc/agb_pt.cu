@@ -1685,6 +1685,36 @@ __global__ void k_vertex_records(const float* pos, const float* nrm, const float
     }
 }
 
+__global__ void k_trace_instances(const int32_t* order, const DevInstance* instances, const DevMesh* meshes, uint32_t n,
+    TraceInstance* out)
+{
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    {
+        const int32_t ii      = order[i];
+        const DevInstance& in = instances[ii];
+        const DevMesh& m      = meshes[in.mesh];
+        TraceInstance t{};
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            t.w2o[r] = make_float4(in.w2o[4 * r], in.w2o[4 * r + 1], in.w2o[4 * r + 2], in.w2o[4 * r + 3]);
+        t.nodes = reinterpret_cast<const float4*>(m.nodes);
+        t.tris  = m.tris;
+        t.root  = m.root;
+        t.inst  = ii;
+        out[i]  = t;
+    }
+}
+
+cudaError_t launchTraceInstances(const int32_t* order, const DevInstance* instances, const DevMesh* meshes,
+    uint32_t count, TraceInstance* out, cudaStream_t stream)
+{
+    if (count == 0)
+        return cudaSuccess;
+    k_trace_instances<<<std::min<uint32_t>((count + 255) / 256, 65535u), 256, 0, stream>>>(order, instances, meshes,
+        count, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launchVertexRecords(const float* positions, const float* normals, const float* texcoords,
     uint32_t vertexCount, float4* verts, cudaStream_t stream)
 {

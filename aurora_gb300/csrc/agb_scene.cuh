@@ -66,6 +66,18 @@ struct DevInstance
     int32_t layerOffset; // into DevScene::layers
 };
 
+// What a ray needs to enter an instance, one record per TLAS leaf slot (five 16-byte loads side by side
+// instead of the chain leaf slot -> instance -> mesh -> root).
+struct TraceInstance
+{
+    float4 w2o[3];       // world-to-object rows
+    const float4* nodes; // the mesh's BVH nodes and triangles
+    const float4* tris;
+    int32_t root;
+    int32_t inst; // instance index
+    int32_t _pad[2];
+};
+
 // Ground plane constants (the GroundPlane struct of GroundPlane.slang; PTGroundPlane.cpp:62-83):
 // the caller's properties plus the tangent frame built from the normal.
 struct DevGroundPlane
@@ -89,7 +101,7 @@ struct DevScene
     const BNode* tlas;
     int32_t tlasRoot;
     int32_t instanceCount;
-    const int32_t* tlasOrder; // instance index per TLAS leaf slot
+    const TraceInstance* traceInst; // per TLAS leaf slot
     const agb_material* materials;
     const agb_material_textures* matTex; // may be null
     int32_t materialCount;

@@ -49,33 +49,46 @@ struct RayHit
     int32_t inst, prim;
 };
 
-AGB_D float sel3(v3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
+// Three-operand minimum / maximum (one instruction each on sm_100 and later).
+AGB_D float fmax3f(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+AGB_D float fmin3f(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
-// Per-ray constants of the watertight test.
+// Per-ray constants of the watertight test.  The axes are rotated so that the direction's largest component
+// comes last: (kx, ky, kz) = (kz + 1, kz + 2, kz) mod 3.  The paper also swaps kx and ky for a negative
+// largest component, to keep the winding; without the swap the edge functions, their sum and the scaled
+// distance all change sign, exactly, and the accepted triangles and their t, u, v are the same.  (One
+// axis index to select by instead of three; with the instance records, 38.2 -> 34.2 ms of traversal for a
+// 1920x1080, 16-sample frame of the large scene type.)
 struct WtRay
 {
-    v3 o;
-    int kx, ky, kz;
+    v3 o; // origin, rotated
+    int kz;
     float Sx, Sy, Sz;
 };
+AGB_D v3 wtRotate(float x, float y, float z, int kz)
+{
+    return kz == 0 ? v3{ y, z, x } : (kz == 1 ? v3{ z, x, y } : v3{ x, y, z });
+}
 AGB_D WtRay wtSetup(v3 o, v3 d)
 {
     WtRay r;
-    r.o      = o;
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     r.kz     = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
-    r.kx     = r.kz + 1 == 3 ? 0 : r.kz + 1;
-    r.ky     = r.kx + 1 == 3 ? 0 : r.kx + 1;
-    float dz = sel3(d, r.kz);
-    if (dz < 0.f)
-    {
-        int t = r.kx;
-        r.kx  = r.ky;
-        r.ky  = t;
-    }
-    r.Sx = __fdiv_rn(sel3(d, r.kx), dz);
-    r.Sy = __fdiv_rn(sel3(d, r.ky), dz);
-    r.Sz = __fdiv_rn(1.f, dz);
+    r.o      = wtRotate(o.x, o.y, o.z, r.kz);
+    const v3 q = wtRotate(d.x, d.y, d.z, r.kz);
+    r.Sx = __fdiv_rn(q.x, q.z);
+    r.Sy = __fdiv_rn(q.y, q.z);
+    r.Sz = __fdiv_rn(1.f, q.z);
     return r;
 }
 
@@ -83,16 +96,15 @@ AGB_D WtRay wtSetup(v3 o, v3 d)
 AGB_D bool wtIntersect(const WtRay& r, float4 a4, float4 b4, float4 c4, float tmin, float tmax,
     bool inclusive, float& t, float& u, float& v)
 {
-    v3 A = v3{ __fsub_rn(a4.x, r.o.x), __fsub_rn(a4.y, r.o.y), __fsub_rn(a4.z, r.o.z) };
-    v3 B = v3{ __fsub_rn(b4.x, r.o.x), __fsub_rn(b4.y, r.o.y), __fsub_rn(b4.z, r.o.z) };
-    v3 C = v3{ __fsub_rn(c4.x, r.o.x), __fsub_rn(c4.y, r.o.y), __fsub_rn(c4.z, r.o.z) };
-    float Akz = sel3(A, r.kz), Bkz = sel3(B, r.kz), Ckz = sel3(C, r.kz);
-    float Ax = __fsub_rn(sel3(A, r.kx), __fmul_rn(r.Sx, Akz));
-    float Ay = __fsub_rn(sel3(A, r.ky), __fmul_rn(r.Sy, Akz));
-    float Bx = __fsub_rn(sel3(B, r.kx), __fmul_rn(r.Sx, Bkz));
-    float By = __fsub_rn(sel3(B, r.ky), __fmul_rn(r.Sy, Bkz));
-    float Cx = __fsub_rn(sel3(C, r.kx), __fmul_rn(r.Sx, Ckz));
-    float Cy = __fsub_rn(sel3(C, r.ky), __fmul_rn(r.Sy, Ckz));
+    const v3 a = wtRotate(a4.x, a4.y, a4.z, r.kz), b = wtRotate(b4.x, b4.y, b4.z, r.kz),
+             c = wtRotate(c4.x, c4.y, c4.z, r.kz);
+    float Akz = __fsub_rn(a.z, r.o.z), Bkz = __fsub_rn(b.z, r.o.z), Ckz = __fsub_rn(c.z, r.o.z);
+    float Ax = __fsub_rn(__fsub_rn(a.x, r.o.x), __fmul_rn(r.Sx, Akz));
+    float Ay = __fsub_rn(__fsub_rn(a.y, r.o.y), __fmul_rn(r.Sy, Akz));
+    float Bx = __fsub_rn(__fsub_rn(b.x, r.o.x), __fmul_rn(r.Sx, Bkz));
+    float By = __fsub_rn(__fsub_rn(b.y, r.o.y), __fmul_rn(r.Sy, Bkz));
+    float Cx = __fsub_rn(__fsub_rn(c.x, r.o.x), __fmul_rn(r.Sx, Ckz));
+    float Cy = __fsub_rn(__fsub_rn(c.y, r.o.y), __fmul_rn(r.Sy, Ckz));
     float U  = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
     float V  = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     float W  = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -103,7 +115,8 @@ AGB_D bool wtIntersect(const WtRay& r, float4 a4, float4 b4, float4 c4, float tm
         V = float(__dsub_rn(__dmul_rn(double(Ax), double(Cy)), __dmul_rn(double(Ay), double(Cx))));
         W = float(__dsub_rn(__dmul_rn(double(Bx), double(Ay)), __dmul_rn(double(By), double(Ax))));
     }
-    if ((U < 0.f || V < 0.f || W < 0.f) && (U > 0.f || V > 0.f || W > 0.f))
+    // Of mixed sign: outside.  (A NaN is left out of both; the determinant then rejects it below.)
+    if (fmin3f(U, V, W) < 0.f && fmax3f(U, V, W) > 0.f)
         return false;
     float det = __fadd_rn(__fadd_rn(U, V), W);
     if (det == 0.f)
@@ -121,22 +134,12 @@ AGB_D bool wtIntersect(const WtRay& r, float4 a4, float4 b4, float4 c4, float tm
 }
 
 // Affine transform of a ray into object space, unrounded-contraction-free so that host and device
-// agree: ((m0 x + m1 y) + m2 z) + m3.
-AGB_D v3 xfPointRn(const float* m, v3 p)
+// agree: one row, (m0 x + m1 y) + m2 z, for points + m3.
+AGB_D float xfRowRn(float4 m, v3 p)
 {
-    return v3{ __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], p.x), __fmul_rn(m[1], p.y)),
-                             __fmul_rn(m[2], p.z)), m[3]),
-        __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[4], p.x), __fmul_rn(m[5], p.y)),
-                      __fmul_rn(m[6], p.z)), m[7]),
-        __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[8], p.x), __fmul_rn(m[9], p.y)),
-                      __fmul_rn(m[10], p.z)), m[11]) };
+    return __fadd_rn(__fadd_rn(__fmul_rn(m.x, p.x), __fmul_rn(m.y, p.y)), __fmul_rn(m.z, p.z));
 }
-AGB_D v3 xfVectorRn(const float* m, v3 v)
-{
-    return v3{ __fadd_rn(__fadd_rn(__fmul_rn(m[0], v.x), __fmul_rn(m[1], v.y)), __fmul_rn(m[2], v.z)),
-        __fadd_rn(__fadd_rn(__fmul_rn(m[4], v.x), __fmul_rn(m[5], v.y)), __fmul_rn(m[6], v.z)),
-        __fadd_rn(__fadd_rn(__fmul_rn(m[8], v.x), __fmul_rn(m[9], v.y)), __fmul_rn(m[10], v.z)) };
-}
+AGB_D float xfRowRn(float4 m, v3 p, float t) { return __fadd_rn(xfRowRn(m, p), t); }
 
 struct SlabRay
 {
@@ -161,19 +164,6 @@ AGB_D SlabRay slabSetup(v3 o, v3 d)
     s.inv  = v3{ rcpApprox(dx), rcpApprox(dy), rcpApprox(dz) };
     s.oinv = v3{ o.x * s.inv.x, o.y * s.inv.y, o.z * s.inv.z };
     return s;
-}
-// Three-operand minimum / maximum (one instruction each on sm_100 and later).
-AGB_D float fmax3f(float a, float b, float c)
-{
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-AGB_D float fmin3f(float a, float b, float c)
-{
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
 }
 // Two child boxes of a node against [tmin, tmax] (tmin >= 0); returns entry distances.
 AGB_D void slab2(const SlabRay& s, float4 c0xy, float4 c1xy, float4 cz, float tmin, float tmax,
@@ -209,10 +199,9 @@ AGB_D void slab2(const SlabRay& s, float4 c0xy, float4 c1xy, float4 cz, float tm
 // Every outer iteration has three phases with uniform work inside each, so the lanes of a warp run
 // the same instructions together:
 //   node phase      lanes step through internal nodes (TLAS or BLAS).  A lane that reaches a BLAS
-//                   leaf parks it (in `leaf`, then `leaf2`) and keeps traversing speculatively
-//                   until it holds kParkLeaves leaves and reaches another; a lane that reaches an
-//                   instance boundary waits.  The phase ends once every lane holds a parked leaf,
-//                   waits at a boundary or has finished.
+//                   leaf parks it and keeps traversing speculatively until it reaches another; a
+//                   lane that reaches an instance boundary waits.  The phase ends once every lane
+//                   holds a parked leaf, waits at a boundary or has finished.
 //   leaf phase      lanes test the triangles of their parked leaves, one triangle per iteration.
 //   boundary phase  lanes at a TLAS leaf enter its instance (object-space ray, watertight and slab
 //                   setup); lanes at kExitInstance return to the world-space ray and the TLAS.
@@ -232,14 +221,8 @@ constexpr int32_t kDone = int32_t(0x80000001);
 // Leaf refs are the negative values above kDone (the two most negative values are the markers).
 AGB_D bool isLeafRef(int32_t ref) { return uint32_t(ref) - uint32_t(kDone + 1) < 0x7fffffffu - 1u; }
 
-#ifndef AGB_TRACE_PARK
-#define AGB_TRACE_PARK 1
-#endif
 #ifndef AGB_NODE_EXIT
 #define AGB_NODE_EXIT 8
-#endif
-#ifndef AGB_NODE_LOAD256
-#define AGB_NODE_LOAD256 1
 #endif
 // One 32-byte read-only load (two float4) per lane: a node is two of them instead of four 16-byte
 // loads, which halves the L1 wavefronts of the divergent node fetches.  p must be 32-byte aligned.
@@ -249,19 +232,15 @@ AGB_D void ldg256(const float4* p, float4& a, float4& b)
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
         : "l"(p));
 }
-#ifndef AGB_SHADOW_PARK
-#define AGB_SHADOW_PARK 2
-#endif
-#ifndef AGB_SHADOW_NODE_EXIT
-#define AGB_SHADOW_NODE_EXIT AGB_NODE_EXIT
-#endif
-// Leaves a lane may park before it stops in the node phase (1 or 2): closest-hit and any-hit rays.
-constexpr int kParkLeavesClosest = AGB_TRACE_PARK;
-constexpr int kParkLeavesAny     = AGB_SHADOW_PARK;
-// The node phase also ends once fewer than this many lanes are still searching for their first
-// leaf while some lane holds a parked leaf (0: only when none is searching).
-constexpr int kNodeExitLanesClosest = AGB_NODE_EXIT;
-constexpr int kNodeExitLanesAny     = AGB_SHADOW_NODE_EXIT;
+// The node phase ends once fewer than this many lanes are still searching for their first leaf while some
+// lane holds a parked leaf (0: only when none is searching).
+constexpr int kNodeExitLanes = AGB_NODE_EXIT;
+// Node steps between two of the warp's votes on whether to go on (a lane takes the later ones only while it
+// is at an internal node).  The kernels issue on 0.7 of the cycles, so instructions are what counts, and
+// the votes and their branches are a good part of a step: closest-hit and shadow rays of a 1920x1080,
+// 16-sample frame of the large scene type 34.2 ms with 1 step, 31.9 with 2, 31.9 with 3.  (Two parked
+// leaves, for either kind of ray, cost more than they give since.)
+constexpr int kNodeSteps = 2;
 
 // A Writer whose kRestart is true is called as write(scene, ray, hit?, hit, tmin) and returns
 // false to trace the same ray again from the tmin it sets (transparent shadows walk the hits
@@ -314,9 +293,6 @@ template <bool kAnyHit, bool kCount, class Loader, class Writer>
 AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32_t* work, const Loader& load,
     const Writer& write, int32_t* stack, int stride, TraceCounters& cnt, bool& overflow)
 {
-    constexpr int kParkLeaves    = kAnyHit ? kParkLeavesAny : kParkLeavesClosest;
-    constexpr int kNodeExitLanes = kAnyHit ? kNodeExitLanesAny : kNodeExitLanesClosest;
-    static_assert(kParkLeaves == 1 || kParkLeaves == 2, "one or two parked leaves");
     const unsigned FULL = 0xffffffffu;
     const int lane      = threadIdx.x & 31;
     bool active = false, exhausted = uint32_t(lane) >= lanes;
@@ -325,7 +301,7 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
     float tmin = 0.f, tmax = 0.f, tmaxRay = 0.f;
     SlabRay sr;
     WtRay wr;
-    int32_t ref = kDone, leaf = 0, leaf2 = 0;
+    int32_t ref = kDone, leaf = 0; // kDone while the lane has no ray
     int sp       = 0;
     int32_t inst = -1;
     const float4* nodes = nullptr;
@@ -370,7 +346,6 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
                     sr       = slabSetup(o, d);
                     ref      = rayRoot(load, s, rayIdx);
                     leaf     = 0;
-                    leaf2    = 0;
                     sp       = 0;
                     inst     = -1;
                     nodes    = reinterpret_cast<const float4*>(s.tlas);
@@ -386,25 +361,17 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
         if (__all_sync(FULL, exhausted))
             break;
 
-        // Node phase: internal nodes only.  A lane stops at a BLAS leaf once it holds kParkLeaves
-        // parked leaves (until then it parks the leaf and goes on speculatively), at an instance
-        // boundary (TLAS leaf or kExitInstance) or at the end of its ray.
+        // Node phase: internal nodes only.  A lane stops at a BLAS leaf once it holds a parked one (until
+        // then it parks the leaf and goes on speculatively), at an instance boundary (TLAS leaf or
+        // kExitInstance) or at the end of its ray.
         for (;;)
         {
-            if (active && inst >= 0 && isLeafRef(ref))
+            if (leaf == 0 && inst >= 0 && isLeafRef(ref))
             {
-                if (leaf == 0)
-                {
-                    leaf = ref;
-                    ref  = pop();
-                }
-                else if (kParkLeaves > 1 && leaf2 == 0)
-                {
-                    leaf2 = ref;
-                    ref   = pop();
-                }
+                leaf = ref;
+                ref  = pop();
             }
-            bool nodeWork      = active && ref >= 0;
+            bool nodeWork      = ref >= 0;
             unsigned searching = __ballot_sync(FULL, nodeWork && leaf == 0);
             if (searching == 0)
                 break;
@@ -412,45 +379,41 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
                 break;
             if (!nodeWork)
                 continue;
-            const float4* np = nodes + 4 * size_t(ref);
-            float4 c0xy, c1xy, cz;
-            int4 refs;
-#if AGB_NODE_LOAD256
-            ldg256(np, c0xy, c1xy);
-            {
-                float4 r4;
+            auto nodeStep = [&]() {
+                const float4* np = nodes + 4 * size_t(ref);
+                float4 c0xy, c1xy, cz, r4;
+                ldg256(np, c0xy, c1xy);
                 ldg256(np + 2, cz, r4);
-                refs = make_int4(__float_as_int(r4.x), __float_as_int(r4.y), __float_as_int(r4.z),
-                    __float_as_int(r4.w));
-            }
-#else
-            c0xy = __ldg(np), c1xy = __ldg(np + 1), cz = __ldg(np + 2);
-            refs = __ldg(reinterpret_cast<const int4*>(np + 3));
-#endif
-            if (kCount)
-                cnt.nodes++;
-            bool h0, h1;
-            float t0, t1;
-            slab2(sr, c0xy, c1xy, cz, tmin, tmax, h0, h1, t0, t1);
-            if (h0 && h1)
-            {
-                if (sp >= kStackSize - 1)
+                const int32_t ref0 = __float_as_int(r4.x), ref1 = __float_as_int(r4.y);
+                if (kCount)
+                    cnt.nodes++;
+                bool h0, h1;
+                float t0, t1;
+                slab2(sr, c0xy, c1xy, cz, tmin, tmax, h0, h1, t0, t1);
+                if (h0 && h1)
                 {
-                    overflow = true;
-                    ref = kDone, leaf = leaf2 = 0, sp = 0;
-                    continue;
+                    if (sp >= kStackSize - 1)
+                    {
+                        overflow = true;
+                        ref = kDone, leaf = 0, sp = 0;
+                        return;
+                    }
+                    push(t0 <= t1 ? ref1 : ref0);
+                    ref = t0 <= t1 ? ref0 : ref1;
                 }
-                push(t0 <= t1 ? refs.y : refs.x);
-                ref = t0 <= t1 ? refs.x : refs.y;
-            }
-            else if (h0 || h1)
-                ref = h0 ? refs.x : refs.y;
-            else
-                ref = pop();
+                else if (h0 || h1)
+                    ref = h0 ? ref0 : ref1;
+                else
+                    ref = pop();
+            };
+            nodeStep();
+#pragma unroll
+            for (int k = 1; k < kNodeSteps; k++)
+                if (ref >= 0)
+                    nodeStep();
         }
 
-        // Leaf phase: one triangle per lane per iteration over the lanes' parked leaves, so lanes
-        // whose leaves hold different triangle counts do not wait for one another leaf by leaf.
+        // Leaf phase: the triangles of the lanes' parked leaves, one per lane per iteration.
         uint32_t cur = 0, end = 0;
         if (leaf != 0)
         {
@@ -459,22 +422,9 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
             end           = cur + (code & 7u) + 1u;
             leaf          = 0;
         }
-        while (__any_sync(FULL, cur < end))
-        {
-            if (cur >= end)
-                continue;
-            const float4* tp = tris + 3 * size_t(cur);
-            float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+        auto testTriangle = [&](float4 a, float4 b, float4 c) {
             if (kCount)
                 cnt.tris++;
-            cur++;
-            if (cur == end && leaf2 != 0)
-            {
-                uint32_t code = uint32_t(~leaf2);
-                cur           = code >> 3;
-                end           = cur + (code & 7u) + 1u;
-                leaf2         = 0;
-            }
             float t, u, v;
             if (wtIntersect(wr, a, b, c, tmin, tmax, !kAnyHit && found, t, u, v))
             {
@@ -493,20 +443,26 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
                 {
                     ref = kDone, sp = 0;
                     cur = end = 0;
-                    leaf2     = 0;
                 }
             }
+        };
+        while (__any_sync(FULL, cur < end))
+        {
+            if (cur >= end)
+                continue;
+            const float4* tp = tris + 3 * size_t(cur++);
+            testTriangle(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2));
         }
 
         // Instance boundaries, taken together by the lanes that reached one.
-        if (active && ref == kExitInstance)
+        if (ref == kExitInstance)
         {
             inst  = -1;
             nodes = reinterpret_cast<const float4*>(s.tlas);
             sr    = slabSetup(o, d);
             ref   = pop();
         }
-        else if (active && inst < 0 && isLeafRef(ref))
+        else if (inst < 0 && isLeafRef(ref))
         {
             // TLAS leaf: one instance (the TLAS is built with single-instance leaves).
             if (sp >= kStackSize - 1)
@@ -516,19 +472,19 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
             }
             else
             {
-                uint32_t first = uint32_t(~ref) >> 3;
-                int32_t ii     = __ldg(s.tlasOrder + first);
-                const DevInstance& in = s.instances[ii];
-                const DevMesh& m      = s.meshes[in.mesh];
+                const float4* ti = reinterpret_cast<const float4*>(s.traceInst + (uint32_t(~ref) >> 3));
+                const float4 m0 = __ldg(ti), m1 = __ldg(ti + 1), m2 = __ldg(ti + 2);
+                const ulonglong2 ptrs = __ldg(reinterpret_cast<const ulonglong2*>(ti + 3));
+                const int2 ids        = __ldg(reinterpret_cast<const int2*>(ti + 4));
                 push(kExitInstance);
-                v3 oo = xfPointRn(in.w2o, o);
-                v3 od = xfVectorRn(in.w2o, d);
+                v3 oo = v3{ xfRowRn(m0, o, m0.w), xfRowRn(m1, o, m1.w), xfRowRn(m2, o, m2.w) };
+                v3 od = v3{ xfRowRn(m0, d), xfRowRn(m1, d), xfRowRn(m2, d) };
                 wr    = wtSetup(oo, od);
                 sr    = slabSetup(oo, od);
-                inst  = ii;
-                nodes = reinterpret_cast<const float4*>(m.nodes);
-                tris  = m.tris;
-                ref   = m.root;
+                inst  = ids.y;
+                nodes = reinterpret_cast<const float4*>(ptrs.x);
+                tris  = reinterpret_cast<const float4*>(ptrs.y);
+                ref   = ids.x;
             }
         }
         if (active && ref == kDone)
