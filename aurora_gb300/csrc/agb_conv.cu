@@ -550,10 +550,18 @@ struct WgradTmaArgs
     int* error;
 };
 
+// Shared memory of one accumulator row of the epilogue: 16 bytes of padding keep its stores free of conflicts.
+template <int N>
+constexpr uint32_t kWgRowBytes = uint32_t(N) * 4u + 16u;
+
 template <int N>
 __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tm0,
     const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tmDy, const WgradTmaArgs a)
 {
+    // Where the TMEM holds two sets of the accumulators, an item sums the halves of its range apart and adds
+    // them at the end: the tensor core's FP32 accumulation loses a little with every unit, so a sum is
+    // kept no longer than half of what one item per SM has to cover.
+    constexpr bool kTwoSets = 6 * N <= 512;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t full[kWgMaxStages], empty[kWgMaxStages], accFull;
     __shared__ uint32_t tmemBase;
@@ -571,6 +579,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
     const int dyIt = item / a.ciTiles; // the item's dy when T == 1
     const int u0   = sp * a.unitsPerItem;
     const int u1   = min(a.numUnits, u0 + a.unitsPerItem);
+    const int mid  = kTwoSets ? u0 + (u1 - u0 + 1) / 2 : u1; // units from here on go to the second set
 
     if (warp == 1)
         tc::tmemAlloc(&tmemBase, 512);
@@ -662,9 +671,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
             // MN-major A and B (bits 15, 16), M = 128, N.
             const uint32_t idesc = tc::idescBf16(128, N) | (1u << 15) | (1u << 16);
             uint32_t it          = 0;
-            bool first           = true;
             for (int u = u0; u < u1; u++, it++)
             {
+                const bool first   = u == u0 || u == mid;
+                const uint32_t acc = tmem + (u < mid ? 0u : 3u * N);
                 const int s       = int(it % uint32_t(S));
                 const uint32_t ph = (it / uint32_t(S)) & 1u;
                 if (!tc::mbarWait(&full[s], ph))
@@ -690,11 +700,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
                         const uint64_t bd    = bDesc0 + ((uint32_t(par) * (N / 16) * kWgSlotB) >> 4);
 #pragma unroll
                         for (int ks = 0; ks < 4; ks++)
-                            tc::mma(tmem + uint32_t(dx * N), ad + ((uint32_t(ks) * 16u * 32u) >> 4),
+                            tc::mma(acc + uint32_t(dx * N), ad + ((uint32_t(ks) * 16u * 32u) >> 4),
                                 bd + ((uint32_t(ks) * 16u * 32u) >> 4), idesc,
                                 (first && par == 0 && ks == 0) ? 0u : 1u);
                     }
-                first = false;
                 tc::commit(&empty[s]);
             }
             tc::commit(&accFull);
@@ -718,23 +727,35 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
             const int dy         = a.T == 3 ? t : dyIt;
             const int ci         = (a.T == 3 ? 0 : ciT * 128) + m % rowsPerTap;
             const bool valid     = t < a.T && ci < a.Cin;
+            // Each thread's rows (one per horizontal tap) go through shared memory - the stages are free once
+            // the MMAs are done - and are added to dW by one bulk reduction each: whole rows of N floats
+            // instead of N / 4 16-byte reductions that each touch half a sector.
+            uint8_t* const rows = smem + size_t(m) * kWgRowBytes<N>;
             for (int dx = 0; dx < 3; dx++)
+            {
+                uint8_t* const row = rows + size_t(dx) * 128 * kWgRowBytes<N>;
                 for (int c0 = 0; c0 < N; c0 += 16)
                 {
-                    uint32_t v[16];
-                    tc::tmemLoad16(tmem + (uint32_t(quad * 32) << 16) + uint32_t(dx * N + c0), v);
+                    uint32_t v[16], v2[16];
+                    const uint32_t col = tmem + (uint32_t(quad * 32) << 16) + uint32_t(dx * N + c0);
+                    tc::tmemLoad16(col, v);
+                    if (mid < u1)
+                        tc::tmemLoad16(col + 3u * N, v2);
                     tc::tmemWaitLoad();
-                    if (valid)
-                    {
-                        float* dst = a.dw + (size_t(dy * 3 + dx) * a.Cin + ci) * a.Cout + coT * N + c0;
+                    if (mid < u1)
 #pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * q),
-                                "f"(__uint_as_float(v[4 * q])), "f"(__uint_as_float(v[4 * q + 1])),
-                                "f"(__uint_as_float(v[4 * q + 2])), "f"(__uint_as_float(v[4 * q + 3]))
-                                         : "memory");
-                    }
+                        for (int q = 0; q < 16; q++)
+                            v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(v2[q]));
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        reinterpret_cast<uint4*>(row)[c0 / 4 + q] =
+                            make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
+                tc::fenceProxyAsync();
+                if (valid)
+                    tc::bulkReduceAdd(a.dw + (size_t(dy * 3 + dx) * a.Cin + ci) * a.Cout + coT * N, row, uint32_t(N) * 4u);
+            }
+            tc::bulkCommitWait();
         }
     }
     tc::fenceBeforeSync();
@@ -926,7 +947,19 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     a.numUnits = c.B * c.H * a.unitsX;
     const int fixedItems = (a.T == 3 ? 1 : 3) * a.ciTiles * a.coTiles;
     const int sms        = smCount > 0 ? smCount : 148;
-    a.splits       = std::max(1, std::min(a.numUnits, (2 * sms + fixedItems - 1) / fixedItems));
+    // A CTA takes a whole SM.  Two items per SM; where the kernel sums two halves of an item apart, two at most
+    // (306 items on 152 SMs take three rounds), or one, if the item is short and its halves no longer than
+    // a sum of the two-item split: every item pays a prologue, a pipeline fill and its reductions into dW
+    // (64 to 64 channels at 4 x 128 x 128, 11 units an item: 20 us against 26), which long items hide.
+    // One sum over a whole item would double the error against 64 bits.
+    const bool twoSets = 6 * a.N <= 512;
+    auto splitsFor     = [&](int items) { return std::max(1, std::min(a.numUnits, items / fixedItems)); };
+    auto perItem       = [&](int splits) { return (a.numUnits + splits - 1) / splits; };
+    const int one = splitsFor(sms), two = splitsFor(2 * sms + fixedItems - 1);
+    if (!twoSets)
+        a.splits = two;
+    else
+        a.splits = (perItem(one) + 1) / 2 <= perItem(two) && perItem(one) <= 32 ? one : splitsFor(2 * sms);
     a.unitsPerItem = (a.numUnits + a.splits - 1) / a.splits;
     a.splits       = (a.numUnits + a.unitsPerItem - 1) / a.unitsPerItem;
     a.numItems     = fixedItems * a.splits;
@@ -950,7 +983,9 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
         m1 = m0;
     if ((e = mapPairs(&md, dy, c.B, c.H, c.W, c.Cout, kWgEntriesB)) != cudaSuccess)
         return e;
-    const size_t smem = std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024);
+    // The stages, or the epilogue's rows (three times 128) in their place.
+    const size_t smem = std::max<size_t>(std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024),
+        size_t(3) * 128 * (size_t(a.N) * 4 + 16));
     auto kern = a.N == 128 ? k_conv_wgrad_tma<128> : a.N == 96 ? k_conv_wgrad_tma<96> : a.N == 64 ? k_conv_wgrad_tma<64>
         : a.N == 48 ? k_conv_wgrad_tma<48> : a.N == 32 ? k_conv_wgrad_tma<32> : k_conv_wgrad_tma<16>;
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)

@@ -106,6 +106,21 @@ __device__ __forceinline__ void bulkLoad(void* dst, const void* src, uint32_t by
                  : "memory");
 }
 
+// Adds `bytes` of FP32 from shared to global memory, elementwise (bulk reduction); dst, src and bytes must be
+// multiples of 16.  The caller's writes to src come before it through fenceProxyAsync.
+__device__ __forceinline__ void bulkReduceAdd(float* dst, const void* src, uint32_t bytes)
+{
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+        "r"(smemAddr(src)), "r"(bytes)
+                 : "memory");
+}
+// Waits until this thread's bulk reductions have been written.
+__device__ __forceinline__ void bulkCommitWait()
+{
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // Tiled tensor copies global -> shared through a tensor map (TMA); completion counted on the
 // mbarrier.  Coordinates are in elements, innermost first; elements outside the tensor read as
 // zero.  The innermost coordinate times the element size must be a multiple of 16 bytes, and dst
