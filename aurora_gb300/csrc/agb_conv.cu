@@ -54,6 +54,7 @@ constexpr uint32_t kRowBytes    = 4352;              // kBoxBytes rounded up to 
 constexpr int kThreads          = 320; // producer, MMA issuer, 8 epilogue warps
 constexpr uint32_t kAccStride   = 256;               // TMEM columns per accumulator buffer
 constexpr int kMaxStages        = 4;
+constexpr int kMaxGradChannels  = 256;               // channels of a dpre0 output
 constexpr size_t kSmemBudget    = 226 * 1024; // of the 227 KB a CTA may have, static shared memory aside
 
 struct ConvTmaArgs
@@ -68,6 +69,9 @@ struct ConvTmaArgs
     int* error;            // set to 1 when a bounded wait runs out
     float* g0;             // data-gradient split (see ConvLaunch)
     float* g1;
+    uint16_t* dpre0;
+    const uint16_t* act0;
+    float* db0;
     int gC0, gUp;
     int B, H, W, Cout, up0, relu;
     int N, nTiles, R, G, G0, stages;
@@ -182,6 +186,67 @@ __device__ __forceinline__ void issueStage(uint32_t aAddr, uint32_t bAddr, uint3
     }
 }
 
+// Two 16-byte loads of 16 BF16 values, masked to where they are positive: the ReLU's gradient of f, rounded to
+// BF16 pairs.
+__device__ __forceinline__ void reluGrad16(const uint16_t* act, const float (&f)[16], uint32_t (&w)[8])
+{
+    const uint4* ap = reinterpret_cast<const uint4*>(act);
+    const uint4 a0 = __ldg(ap), a1 = __ldg(ap + 1);
+    const uint32_t y[8] = { a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w };
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+    {
+        const float lo = __uint_as_float(y[i] << 16) > 0.f ? f[2 * i] : 0.f;
+        const float hi = __uint_as_float(y[i] & 0xFFFF0000u) > 0.f ? f[2 * i + 1] : 0.f;
+        const __nv_bfloat162 h2 = __floats2bfloat162_rn(lo, hi);
+        w[i]                    = *reinterpret_cast<const uint32_t*>(&h2);
+    }
+}
+
+__device__ __forceinline__ void addBf16(float (&sum)[16], const uint32_t (&w)[8])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+    {
+        sum[2 * i] += __uint_as_float(w[i] << 16);
+        sum[2 * i + 1] += __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ void stFloat16(float* p, const float (&f)[16])
+{
+    uint32_t w0[8], w1[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+    {
+        w0[i] = __float_as_uint(f[i]);
+        w1[i] = __float_as_uint(f[8 + i]);
+    }
+    st256(p, w0);
+    st256(p + 8, w1);
+}
+
+// Adds the warp's sums of 16 values per lane to dst[0 .. 16) (shared memory): halves of the values are
+// exchanged with the lane across, so 16 shuffles leave every channel's sum in a lane pair.
+__device__ __forceinline__ void warpAddChannels(float (&v)[16], float* dst, int lane)
+{
+#pragma unroll
+    for (int n = 8; n >= 1; n >>= 1)
+    {
+        const int mask  = 2 * n;
+        const bool high = (lane & mask) != 0;
+#pragma unroll
+        for (int k = 0; k < n; k++)
+        {
+            const float give = high ? v[k] : v[k + n];
+            const float keep = high ? v[k + n] : v[k];
+            v[k]             = keep + __shfl_xor_sync(0xffffffffu, give, mask);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 1) == 0)
+        atomicAdd(dst + (lane >> 1), v[0]);
+}
+
 template <int N, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_constant__ CUtensorMap tm0,
     const __grid_constant__ CUtensorMap tm1, const ConvTmaArgs a)
@@ -190,11 +255,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t full[kMaxStages], empty[kMaxStages], accFull[2], accEmpty[2], drain;
     __shared__ uint32_t tmemBase;
+    __shared__ float biasGrad[SPLIT ? kMaxGradChannels : 1]; // this CTA's share of db0
     const int tid  = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
     const int S    = a.stages;
 
+    if (SPLIT)
+        for (int c = tid; c < kMaxGradChannels; c += kThreads)
+            biasGrad[c] = 0.f;
     if (warp == 1)
         tc::tmemAlloc(&tmemBase, 2 * kAccStride);
     if (tid == 0)
@@ -389,7 +458,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                     for (int i = 0; i < 16; i++)
                         bv[i] = 0.f;
                 }
-                float psum[16], gsum[16];
+                float psum[16], gsum[16], bsum[16];
+                if (split)
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        bsum[i] = 0.f;
                 const int cch   = cb + c0; // output channel of the chunk
                 const bool toG0 = split && cch < a.gC0;
 #pragma unroll
@@ -442,25 +515,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                     {
                         if (toG0 && a.gUp)
                         {
-                            // 2x2 block sum ((x00 + x01) + x10) + x11, added below.
+                            // 2x2 block sum ((x00 + x01) + x10) + x11, stored below.
 #pragma unroll
                             for (int i = 0; i < 16; i++)
                                 gsum[i] = acc == 0 ? f[i] : gsum[i] + f[i];
                         }
+                        else if (st && toG0 && a.dpre0)
+                        {
+                            reluGrad16(a.act0 + px * a.gC0 + cch, f, w);
+                            st256(a.dpre0 + px * a.gC0 + cch, w);
+                            addBf16(bsum, w);
+                        }
                         else if (st)
                         {
-                            float* g   = toG0 ? a.g0 + px * a.gC0 + cch : a.g1 + px * (a.Cout - a.gC0) + (cch - a.gC0);
-                            float4* g4 = reinterpret_cast<float4*>(g);
-#pragma unroll
-                            for (int i = 0; i < 4; i++)
-                            {
-                                float4 o = g4[i];
-                                o.x += f[4 * i];
-                                o.y += f[4 * i + 1];
-                                o.z += f[4 * i + 2];
-                                o.w += f[4 * i + 3];
-                                g4[i] = o;
-                            }
+                            float* g = toG0 ? a.g0 + px * a.gC0 + cch : a.g1 + px * (a.Cout - a.gC0) + (cch - a.gC0);
+                            stFloat16(g, f);
                         }
                     }
                     if (a.pool)
@@ -477,19 +546,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                 }
                 if (split && toG0 && a.gUp && colOk && q.y0 + r + 1 < a.H)
                 {
-                    const size_t pp = (size_t(q.b) * (a.H >> 1) + ((q.y0 + r) >> 1)) * W2 + j;
-                    float4* g4      = reinterpret_cast<float4*>(a.g0 + pp * a.gC0 + cch);
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
+                    const size_t at = ((size_t(q.b) * (a.H >> 1) + ((q.y0 + r) >> 1)) * W2 + j) * a.gC0 + cch;
+                    if (a.dpre0)
                     {
-                        float4 o = g4[i];
-                        o.x += gsum[4 * i];
-                        o.y += gsum[4 * i + 1];
-                        o.z += gsum[4 * i + 2];
-                        o.w += gsum[4 * i + 3];
-                        g4[i] = o;
+                        uint32_t w[8];
+                        reluGrad16(a.act0 + at, gsum, w);
+                        st256(a.dpre0 + at, w);
+                        addBf16(bsum, w);
                     }
+                    else
+                        stFloat16(a.g0 + at, gsum);
                 }
+                if (split && toG0 && a.dpre0)
+                    warpAddChannels(bsum, biasGrad + cch, lane);
                 if (a.pool && colOk && q.y0 + r + 1 < a.H)
                 {
                     uint32_t w[8];
@@ -512,6 +581,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
     tc::fenceBeforeSync();
     __syncthreads();
     tc::fenceAfterSync();
+    if (SPLIT && a.dpre0)
+        for (int c = tid; c < a.gC0; c += kThreads)
+            atomicAdd(a.db0 + c, biasGrad[c]);
     if (warp == 1)
         tc::tmemDealloc(tmem, 2 * kAccStride);
     if (!ok)
@@ -880,8 +952,16 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     a.g1    = c.grad1;
     a.gC0   = c.gradC0;
     a.gUp   = c.gradUp;
-    if ((c.grad0 || c.grad1) && (c.gradC0 % 16 || (c.gradUp && c.H % 2) ||
-                                    ((reinterpret_cast<uintptr_t>(c.grad0) | reinterpret_cast<uintptr_t>(c.grad1)) & 15u)))
+    a.dpre0 = c.dpre0;
+    a.act0  = c.act0;
+    a.db0   = c.db0;
+    const bool split = c.grad0 || c.grad1 || c.dpre0;
+    if (split &&
+        (c.gradC0 % 16 || (c.gradUp && c.H % 2) || (c.gradC0 > 0 && !c.grad0 && !c.dpre0) ||
+            (c.gradC0 < c.Cout && !c.grad1) || (c.dpre0 && (!c.act0 || !c.db0 || c.gradC0 > kMaxGradChannels)) ||
+            ((reinterpret_cast<uintptr_t>(c.grad0) | reinterpret_cast<uintptr_t>(c.grad1) |
+                 reinterpret_cast<uintptr_t>(c.dpre0)) & 31u) ||
+            (reinterpret_cast<uintptr_t>(c.act0) & 15u)))
         return cudaErrorInvalidValue;
     a.B = c.B, a.H = c.H, a.W = c.W, a.Cout = c.Cout, a.up0 = c.up0, a.relu = c.relu;
     a.N      = convTileChannels(c.Cout);
@@ -917,7 +997,6 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     // At least half of the SM's shared memory, so that one CTA (with all 512 TMEM columns) runs
     // per SM.
     const size_t smem = std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024);
-    const bool split = c.grad0 || c.grad1;
     auto kern        = split ? (a.N == 64 ? k_conv3x3_tma<64, true> : a.N == 32 ? k_conv3x3_tma<32, true> : k_conv3x3_tma<16, true>)
                              : (a.N == 64 ? k_conv3x3_tma<64, false> : a.N == 32 ? k_conv3x3_tma<32, false> : k_conv3x3_tma<16, false>);
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)

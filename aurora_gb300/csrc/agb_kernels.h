@@ -181,13 +181,19 @@ struct ConvLaunch
     // c = 0..2 (radianceInput: the BF16 features, 16 per pixel, log1p noisy radiance in 0..2).
     float* radiance                = nullptr;
     const uint16_t* radianceInput  = nullptr;
-    // Data-gradient split (the FP32 result is added, not stored): output channels [0, gradC0) go
-    // to grad0 - summed over 2x2 blocks into half resolution when gradUp (the gradient of a
-    // nearest upsample) -, channels [gradC0, Cout) to grad1 at full resolution.
+    // Data-gradient split: output channels [0, gradC0) are the gradient of the layer's first input - summed
+    // over 2x2 blocks into half resolution when gradUp (the gradient of a nearest upsample) -, channels
+    // [gradC0, Cout) that of its second one, stored to grad1 (FP32, full resolution).  The first goes to grad0
+    // (FP32) or, where the input is the ReLU output act0 (BF16) of another layer and has no other
+    // consumer, straight to that layer's pre-activation gradient: dpre0 = bf16(gradient x (act0 > 0)),
+    // and db0[c] += the sum over pixels of dpre0.
     float* grad0 = nullptr;
     float* grad1 = nullptr;
     int gradC0   = 0;
     int gradUp   = 0;
+    uint16_t* dpre0      = nullptr;
+    const uint16_t* act0 = nullptr;
+    float* db0           = nullptr;
 };
 // W even (and H even with up0 or pool), outputs 32-byte aligned; cudaErrorInvalidValue otherwise.
 cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st);
@@ -267,8 +273,7 @@ private:
     uint16_t* act_[kActs] = {};
     float* grad_[kActs]   = {};
     float* out32_ = nullptr;
-    float* gOut_  = nullptr;
-    uint16_t* dpre_        = nullptr;
+    uint16_t* dpre_[2]     = {};
     const uint16_t* input_ = nullptr;
     int B_ = 0, H_ = 0, W_ = 0;
     long step_ = 0;

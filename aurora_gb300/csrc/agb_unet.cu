@@ -2,8 +2,9 @@
 // level, 2x2 average pooling down, nearest 2x upsampling up with skip concatenation, ReLU) over 16
 // input feature channels, trained with an L1 loss and Adam.  Every convolution - forward, data
 // gradient and weight gradient - runs on the tcgen05 tensor cores (agb_denoise.cu) with BF16
-// operands and FP32 accumulation; activations are stored in BF16, gradients between layers are
-// accumulated in FP32, the master weights and Adam moments are FP32.
+// operands and FP32 accumulation; activations are stored in BF16, gradients between layers are FP32
+// until they are rounded once, to the BF16 pre-activation gradient of the layer before (in the data
+// gradient's epilogue where an activation has one consumer), the master weights and Adam moments are FP32.
 //
 // Prediction: log1p(radiance) = log1p(noisy input) + network output (channels 0-2), i.e. the network
 // learns a residual correction in log space.
@@ -37,8 +38,8 @@ inline unsigned gridFor(long n, int block = 256)
 #endif
 // The gradient of one layer's pre-activation and of its bias, from the gradient of its output:
 //   dPre[p][c] = bf16((g[p][c] + 0.25 * gp[p / 2x2][c]) * (y[p][c] > 0)),  db[c] += sum_p dPre[p][c]
-// gp (the gradient of the 2x2 average pool of y, H/2 x W/2) and y (ReLU) are optional; the bias
-// gradient sums the BF16-rounded values the weight gradient uses.  Thread i handles channels
+// with gp the gradient of the 2x2 average pool of y (H/2 x W/2): the skip activations, which have two
+// consumers.  The bias gradient sums the BF16-rounded values the weight gradient uses.  Thread i handles channels
 // 8 (i % G8) .. + 7 of pixel i / G8; the grid stride is a multiple of 256 and so of G8 (C / 8 divides
 // 256), so a thread keeps its channel group and the block reduces per channel in shared memory.
 __global__ void __launch_bounds__(256) k_preact_grad(const float4* g, const float4* gp, const uint4* y, uint4* dpre,
@@ -53,32 +54,26 @@ __global__ void __launch_bounds__(256) k_preact_grad(const float4* g, const floa
     {
         const float4 g0 = g[2 * i], g1 = g[2 * i + 1];
         float v[8]      = { g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w };
-        if (gp)
-        {
-            const long pix = i / G8;
-            const int x    = int(pix % W);
-            const long r   = pix / W;
-            const int yy   = int(r % H);
-            const long b   = r / H;
-            const long q   = ((b * (H / 2) + yy / 2) * (W / 2) + x / 2) * G8 + (i - pix * G8);
-            const float4 p0 = gp[2 * q], p1 = gp[2 * q + 1];
-            const float pv[8] = { p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w };
+        const long pix = i / G8;
+        const int x    = int(pix % W);
+        const long r   = pix / W;
+        const int yy   = int(r % H);
+        const long b   = r / H;
+        const long q   = ((b * (H / 2) + yy / 2) * (W / 2) + x / 2) * G8 + (i - pix * G8);
+        const float4 p0 = gp[2 * q], p1 = gp[2 * q + 1];
+        const float pv[8] = { p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w };
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-                v[k] += 0.25f * pv[k];
-        }
-        if (y)
-        {
-            const uint4 yv      = y[i];
-            const uint32_t w[4] = { yv.x, yv.y, yv.z, yv.w };
+        for (int k = 0; k < 8; k++)
+            v[k] += 0.25f * pv[k];
+        const uint4 yv      = y[i];
+        const uint32_t w[4] = { yv.x, yv.y, yv.z, yv.w };
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-            {
-                if (!(__uint_as_float(w[k] << 16) > 0.f))
-                    v[2 * k] = 0.f;
-                if (!(__uint_as_float(w[k] & 0xFFFF0000u) > 0.f))
-                    v[2 * k + 1] = 0.f;
-            }
+        for (int k = 0; k < 4; k++)
+        {
+            if (!(__uint_as_float(w[k] << 16) > 0.f))
+                v[2 * k] = 0.f;
+            if (!(__uint_as_float(w[k] & 0xFFFF0000u) > 0.f))
+                v[2 * k + 1] = 0.f;
         }
         uint32_t o[4];
 #pragma unroll
@@ -103,33 +98,54 @@ __global__ void __launch_bounds__(256) k_preact_grad(const float4* g, const floa
     }
 }
 
-// L1 loss on log1p(radiance): prediction = out32[p][c] + log1p input (feature channel c), target
-// RGBA FP32.  g (P x 16) = d loss / d out32; loss += sum |pred - log1p(target)| * scale.
-__global__ void k_l1_loss(const float* out32, const uint16_t* x, const float* target, float* g, float* loss,
-    long P, float scale)
+// L1 loss on log1p(radiance): prediction = out32[p][c] + log1p input (feature channel c), target RGBA FP32.
+// dpre (P x 16) = bf16(d loss / d out32), the output layer's pre-activation gradient (it has no ReLU), db += its
+// sums; loss += sum |pred - log1p(target)| * scale.
+__global__ void __launch_bounds__(256) k_l1_loss(const float4* out32, const uint16_t* x, const float4* target,
+    uint4* dpre, float* db, float* loss, long P, float scale)
 {
-    float acc = 0.f;
-    for (long p = blockIdx.x * long(blockDim.x) + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x)
+    __shared__ float part[8][4];
+    float acc[4] = {}; // loss, then the three channels' gradients
+    const uint16_t up = tobf(scale), down = tobf(-scale);
+    for (long p = blockIdx.x * 256L + threadIdx.x; p < P; p += long(gridDim.x) * 256)
     {
+        const float4 o = out32[4 * p], t4 = target[p];
+        const uint2 xv = *reinterpret_cast<const uint2*>(x + 16 * p);
+        const float in[3]   = { bf(uint16_t(xv.x)), bf(uint16_t(xv.x >> 16)), bf(uint16_t(xv.y)) };
+        const float pred[3] = { o.x + in[0], o.y + in[1], o.z + in[2] };
+        const float tv[3]   = { t4.x, t4.y, t4.z };
+        uint16_t g[3];
 #pragma unroll
-        for (int c = 0; c < 16; c++)
+        for (int c = 0; c < 3; c++)
         {
-            float gv = 0.f;
-            if (c < 3)
-            {
-                float pred = out32[p * 16 + c] + bf(x[p * 16 + c]);
-                float t    = log1pf(fmaxf(target[p * 4 + c], 0.f));
-                float d    = pred - t;
-                acc += fabsf(d);
-                gv = d > 0.f ? scale : (d < 0.f ? -scale : 0.f);
-            }
-            g[p * 16 + c] = gv;
+            const float d = pred[c] - log1pf(fmaxf(tv[c], 0.f));
+            acc[0] += fabsf(d);
+            g[c] = d > 0.f ? up : (d < 0.f ? down : uint16_t(0));
+            acc[1 + c] += bf(g[c]);
         }
+        dpre[2 * p]     = make_uint4(uint32_t(g[0]) | (uint32_t(g[1]) << 16), g[2], 0u, 0u);
+        dpre[2 * p + 1] = make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0)
-        atomicAdd(loss, acc * scale);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+        for (int o = 16; o > 0; o >>= 1)
+            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (lane == 0)
+            part[warp][k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4)
+    {
+        float sum = 0.f;
+        for (int w = 0; w < 8; w++)
+            sum += part[w][threadIdx.x];
+        if (threadIdx.x == 0)
+            atomicAdd(loss, sum * scale);
+        else
+            atomicAdd(db + threadIdx.x - 1, sum);
+    }
 }
 
 __global__ void k_adam(float* w, const float* g, float* m, float* v, long n, float lr, float b1, float b2,
@@ -351,7 +367,7 @@ cudaError_t UnetDenoiser::repack()
 
 cudaError_t UnetDenoiser::ensureShape(int B, int H, int W, bool training)
 {
-    if (B == B_ && H == H_ && W == W_ && (!training || grad_[A_E0A]))
+    if (B == B_ && H == H_ && W == W_ && (!training || grad_[A_S0]))
         return cudaSuccess;
     dropGraphs(); // they name the buffers freed here
     for (void* p : shapeAllocs_)
@@ -362,8 +378,8 @@ cudaError_t UnetDenoiser::ensureShape(int B, int H, int W, bool training)
         act_[a]  = nullptr;
         grad_[a] = nullptr;
     }
-    out32_ = gOut_ = nullptr;
-    dpre_  = nullptr;
+    out32_   = nullptr;
+    dpre_[0] = dpre_[1] = nullptr;
     B_ = H_ = W_ = 0;
     cudaError_t e;
     size_t maxDpre = 0;
@@ -372,7 +388,9 @@ cudaError_t UnetDenoiser::ensureShape(int B, int H, int W, bool training)
         size_t n = pixels(B, H, W, kActLevel[a]) * kActChannels[a];
         if ((e = alloc(reinterpret_cast<void**>(&act_[a]), n * 2, shapeAllocs_)) != cudaSuccess)
             return e;
-        if (training && (e = alloc(reinterpret_cast<void**>(&grad_[a]), n * 4, shapeAllocs_)) != cudaSuccess)
+        // FP32 gradients of the skip activations and their pools; the others go straight to BF16.
+        const bool kept = a == A_S0 || a == A_P0 || a == A_S1 || a == A_P1 || a == A_S2 || a == A_P2;
+        if (training && kept && (e = alloc(reinterpret_cast<void**>(&grad_[a]), n * 4, shapeAllocs_)) != cudaSuccess)
             return e;
     }
     size_t p0 = pixels(B, H, W, 0);
@@ -385,9 +403,9 @@ cudaError_t UnetDenoiser::ensureShape(int B, int H, int W, bool training)
             size_t pl = pixels(B, H, W, kLayerDefs[i].level);
             maxDpre   = std::max(maxDpre, pl * layerCout(i));
         }
-        if ((e = alloc(reinterpret_cast<void**>(&gOut_), p0 * 16 * 4, shapeAllocs_)) != cudaSuccess ||
-            (e = alloc(reinterpret_cast<void**>(&dpre_), maxDpre * 2, shapeAllocs_)) != cudaSuccess)
-            return e;
+        for (uint16_t*& d : dpre_)
+            if ((e = alloc(reinterpret_cast<void**>(&d), maxDpre * 2, shapeAllocs_)) != cudaSuccess)
+                return e;
     }
     B_ = B;
     H_ = H;
@@ -527,49 +545,59 @@ cudaError_t UnetDenoiser::backward(const float* target)
     if ((e = cudaMemsetAsync(grads_, 0, nParams_ * 4, stream_)) != cudaSuccess ||
         (e = cudaMemsetAsync(loss_, 0, 4, stream_)) != cudaSuccess)
         return e;
-    for (int a = 1; a < A_COUNT; a++)
-        if ((e = cudaMemsetAsync(grad_[a], 0, pixels(B_, H_, W_, kActLevel[a]) * kActChannels[a] * 4, stream_)) !=
-            cudaSuccess)
-            return e;
     long P0 = long(pixels(B_, H_, W_, 0));
-    k_l1_loss<<<gridFor(P0), 256, 0, stream_>>>(out32_, input_, target, gOut_, loss_, P0, 1.f / float(P0 * 3));
+    // Two pre-activation gradients in turn: the layer's, and the one its data gradient leaves for the layer before.
+    int cur = 0;
+    k_l1_loss<<<unsigned(std::min<long>((P0 + 255) / 256, 4L * smCount_)), 256, 0, stream_>>>(
+        reinterpret_cast<const float4*>(out32_), input_, reinterpret_cast<const float4*>(target),
+        reinterpret_cast<uint4*>(dpre_[cur]), grads_ + bOff_[kLayers - 1], loss_, P0, 1.f / float(P0 * 3));
     for (int i = kLayers - 1; i >= 0; i--)
     {
         const LayerDef& L = kLayerDefs[i];
         const int cin = layerCin(i), cout = layerCout(i);
         const long Pl = long(pixels(B_, H_, W_, L.level));
-        const float* gy = L.out >= 0 ? grad_[L.out] : gOut_;
         // The 2x2 pools of layers 1, 3 and 5 (S -> P): their gradient reaches S here, at half
-        // resolution, beside the gradient from the skip connection.
-        const bool pooled = i == 1 || i == 3 || i == 5;
-        const long n8     = Pl * cout / 8;
-        k_preact_grad<<<unsigned(std::min<long>((n8 + 255) / 256, long(AGB_PREACT_BLOCKS_PER_SM) * smCount_)), 256, 0,
-            stream_>>>(
-            reinterpret_cast<const float4*>(gy), pooled ? reinterpret_cast<const float4*>(grad_[L.out + 1]) : nullptr,
-            L.relu ? reinterpret_cast<const uint4*>(act_[L.out]) : nullptr, reinterpret_cast<uint4*>(dpre_),
-            grads_ + bOff_[i], B_, H_ >> L.level, W_ >> L.level, cout);
+        // resolution, beside the gradient from the skip connection.  Every other layer's output has one
+        // consumer, whose data gradient has left this layer's pre-activation gradient.
+        if (i == 1 || i == 3 || i == 5)
+        {
+            const long n8 = Pl * cout / 8;
+            k_preact_grad<<<unsigned(std::min<long>((n8 + 255) / 256, long(AGB_PREACT_BLOCKS_PER_SM) * smCount_)), 256, 0,
+                stream_>>>(reinterpret_cast<const float4*>(grad_[L.out]),
+                reinterpret_cast<const float4*>(grad_[L.out + 1]), reinterpret_cast<const uint4*>(act_[L.out]),
+                reinterpret_cast<uint4*>(dpre_[cur]), grads_ + bOff_[i], B_, H_ >> L.level, W_ >> L.level, cout);
+        }
         ConvLaunch c = layerLaunch(i, input_);
-        if ((e = launchConvWgrad(c, dpre_, grads_ + wOff_[i], smCount_, stream_)) != cudaSuccess)
+        if ((e = launchConvWgrad(c, dpre_[cur], grads_ + wOff_[i], smCount_, stream_)) != cudaSuccess)
             return e;
         if (i > 0)
         {
-            // dX = the convolution of dPre with the flipped weights, added straight into the
-            // gradients of the layer's inputs (the upsampled one summed over 2x2 blocks).
+            // dX = the convolution of dPre with the flipped weights: the gradient of the first input (the
+            // upsampled one summed over 2x2 blocks) as the pre-activation gradient of the layer that
+            // made it, or in FP32 if a pool did; the gradient of the skip in FP32.
             ConvLaunch d{};
-            d.in0    = dpre_;
+            d.in0    = dpre_[cur];
             d.wpack  = packFlip_ + packOff_[i];
             d.B      = B_;
             d.H      = c.H;
             d.W      = c.W;
             d.C0     = cout;
             d.Cout   = cin;
-            d.grad0  = grad_[L.in0];
+            if (L.in0 == A_P0 || L.in0 == A_P1 || L.in0 == A_P2)
+                d.grad0 = grad_[L.in0];
+            else
+            {
+                d.dpre0 = dpre_[cur ^ 1];
+                d.act0  = act_[L.in0];
+                d.db0   = grads_ + bOff_[i - 1];
+            }
             d.grad1  = L.in1 >= 0 ? grad_[L.in1] : nullptr;
             d.gradC0 = c.C0;
             d.gradUp = L.up0;
             if ((e = launchConv3x3(d, stream_)) != cudaSuccess)
                 return e;
         }
+        cur ^= 1;
     }
     return cudaGetLastError();
 }
