@@ -804,19 +804,6 @@ __global__ void k_reorder_tris(const float* positions, const uint32_t* indices, 
     }
 }
 
-cudaError_t growScratch(void** p, size_t& cap, size_t bytes)
-{
-    if (cap >= bytes)
-        return cudaSuccess;
-    cudaFree(*p);
-    *p  = nullptr;
-    cap = 0;
-    cudaError_t r = cudaMalloc(p, bytes);
-    if (r == cudaSuccess)
-        cap = bytes;
-    return r;
-}
-
 // The large nodes' arrays for n primitives, carved out of one allocation (each level's, twice).
 struct BigArrays
 {
@@ -848,18 +835,37 @@ BigArrays carveBig(void* base, size_t n)
     return b;
 }
 
-// Scratch for n primitives (their boxes are written into s.boxes by the caller): order arrays, the large
-// nodes' arrays (tasksA) and the subtree list (tasksB: every split may leave one).
+// Scratch for n primitives in one allocation: their boxes (written by the caller), order arrays, the large
+// nodes' arrays, the subtree list (every split may leave one) and the counters.
 cudaError_t reserve(GpuBvhScratch& s, size_t n)
 {
-    cudaError_t e;
-    if ((e = growScratch(reinterpret_cast<void**>(&s.boxes), s.boxesBytes, n * 24)) != cudaSuccess ||
-        (e = growScratch(reinterpret_cast<void**>(&s.order), s.orderBytes, n * 4)) != cudaSuccess ||
-        (e = growScratch(reinterpret_cast<void**>(&s.scratch), s.scratchBytes, n * 4)) != cudaSuccess ||
-        (e = growScratch(&s.tasksA, s.tasksABytes, carveBig(nullptr, n).bytes)) != cudaSuccess ||
-        (e = growScratch(&s.tasksB, s.tasksBBytes, (n + 2) * sizeof(BuildTask))) != cudaSuccess ||
-        (e = growScratch(&s.counters, s.countersBytes, 64)) != cudaSuccess)
-        return e;
+    const size_t sizes[6] = { n * 24, n * 4, n * 4, carveBig(nullptr, n).bytes, (n + 2) * sizeof(BuildTask),
+        BC_COUNT * sizeof(uint32_t) };
+    size_t total = 0;
+    for (size_t b : sizes)
+        total += (b + 255) & ~size_t(255);
+    if (s.arraysBytes < total)
+    {
+        cudaFree(s.arrays);
+        s.arrays      = nullptr;
+        s.arraysBytes = 0;
+        const cudaError_t e = cudaMalloc(&s.arrays, total);
+        if (e != cudaSuccess)
+            return e;
+        s.arraysBytes = total;
+    }
+    char* at  = static_cast<char*>(s.arrays);
+    auto take = [&](int k) {
+        void* p = at;
+        at += (sizes[k] + 255) & ~size_t(255);
+        return p;
+    };
+    s.boxes    = static_cast<float*>(take(0));
+    s.order    = static_cast<uint32_t*>(take(1));
+    s.scratch  = static_cast<uint32_t*>(take(2));
+    s.big      = take(3);
+    s.subtrees = take(4);
+    s.counters = take(5);
     return cudaSuccess;
 }
 
@@ -875,8 +881,8 @@ cudaError_t buildLevels(uint32_t n, uint32_t leafMax, int maxDepth, GpuBvhScratc
     unsigned g = unsigned(std::min<size_t>((size_t(n) + 255) / 256, 4096));
     k_iota<<<g, 256, 0, st>>>(s.order, n);
     uint32_t* cnt   = static_cast<uint32_t*>(s.counters);
-    BuildTask* sub  = static_cast<BuildTask*>(s.tasksB);
-    BigArrays big   = carveBig(s.tasksA, n);
+    BuildTask* sub  = static_cast<BuildTask*>(s.subtrees);
+    BigArrays big   = carveBig(s.big, n);
     k_bvh_begin<<<1, kChunkThreads, 0, st>>>(n, cnt, big.tasks[0], big.chunkTask[0], big.nodes[0], sub);
     const bool large = n > uint32_t(kSub);
     // Large nodes of the level, their chunks, subtrees so far.
@@ -953,12 +959,7 @@ cudaError_t buildTlasGpu(const float* boxesHost, uint32_t count, int maxDepth, G
 void freeGpuBvhScratch(GpuBvhScratch& s)
 {
     cudaFree(s.nodes);
-    cudaFree(s.boxes);
-    cudaFree(s.order);
-    cudaFree(s.scratch);
-    cudaFree(s.tasksA);
-    cudaFree(s.tasksB);
-    cudaFree(s.counters);
+    cudaFree(s.arrays);
     s = GpuBvhScratch();
 }
 

@@ -6,9 +6,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "agb_kernels.h"
@@ -47,21 +49,30 @@ agb_status cudaFail(cudaError_t e, const char* what)
             return cudaFail(e_, what);                                                             \
     } while (0)
 
-// A device allocation owned by the context.
+// A device allocation owned by the context, or (view) a part of one that another buffer owns.
 struct DevBuf
 {
     void* ptr    = nullptr;
     size_t bytes = 0;
+    bool part    = false;
     DevBuf()     = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void release()
     {
-        if (ptr)
+        if (ptr && !part)
             cudaFree(ptr);
         ptr   = nullptr;
         bytes = 0;
+        part  = false;
+    }
+    void view(void* p, size_t n)
+    {
+        release();
+        ptr   = p;
+        bytes = n;
+        part  = true;
     }
     cudaError_t ensure(size_t n)
     {
@@ -84,8 +95,31 @@ struct DevBuf
     }
 };
 
+// Carves one allocation into buffers (256-byte steps): each cudaMalloc / cudaFree pair costs about 40 us of
+// host time, and a scene's arrays are made and freed together.
+cudaError_t ensureTogether(DevBuf& whole, std::initializer_list<std::pair<DevBuf*, size_t>> parts)
+{
+    size_t total = 0;
+    for (const auto& p : parts)
+        total += (p.second + 255) & ~size_t(255);
+    for (const auto& p : parts)
+        p.first->release();
+    const cudaError_t e = whole.ensure(total);
+    if (e != cudaSuccess)
+        return e;
+    char* at = whole.as<char>();
+    for (const auto& p : parts)
+    {
+        if (p.second)
+            p.first->view(at, p.second);
+        at += (p.second + 255) & ~size_t(255);
+    }
+    return cudaSuccess;
+}
+
 struct Geometry
 {
+    DevBuf arrays; // holds the six below it that are known before the build
     DevBuf positions, normals, texcoords, verts, indices, tris, nodes;
     DevMesh mesh{};
     uint32_t nodeCount = 0;
@@ -169,7 +203,9 @@ struct agb_context
     WaveBuffers wb{};
     // Accumulation.
     uint32_t accW = 0, accH = 0;
+    DevBuf accArrays; // holds the five below
     DevBuf accMean, accSum, accComp, lastSample, accMoments;
+    DevBuf post32, post8; // post-processing outputs before they are read back
     // Denoising AOVs of the last render that enabled them (accW x accH).
     DevBuf aovDepth, aovNormal, aovAlbedo, aovMotion;
     bool aovValid = false;
@@ -313,11 +349,11 @@ agb_status ensureAccum(agb_context* ctx, uint32_t W, uint32_t H)
     if (ctx->accW == W && ctx->accH == H && ctx->accMean.ptr)
         return AGB_OK;
     size_t n = size_t(W) * H;
-    AGB_CUDA(ctx->accMean.ensure(n * sizeof(float4)), "allocate accumulation");
-    AGB_CUDA(ctx->accSum.ensure(n * sizeof(float4)), "allocate accumulation");
-    AGB_CUDA(ctx->accComp.ensure(n * sizeof(float4)), "allocate accumulation");
-    AGB_CUDA(ctx->lastSample.ensure(n * sizeof(float4)), "allocate accumulation");
-    AGB_CUDA(ctx->accMoments.ensure(n * sizeof(float2)), "allocate accumulation");
+    AGB_CUDA(ensureTogether(ctx->accArrays,
+                 { { &ctx->accMean, n * sizeof(float4) }, { &ctx->accSum, n * sizeof(float4) },
+                     { &ctx->accComp, n * sizeof(float4) }, { &ctx->lastSample, n * sizeof(float4) },
+                     { &ctx->accMoments, n * sizeof(float2) } }),
+        "allocate accumulation");
     AGB_CUDA(cudaMemsetAsync(ctx->accMoments.ptr, 0, n * sizeof(float2), ctx->stream), "clear");
     AGB_CUDA(cudaMemsetAsync(ctx->accMean.ptr, 0, n * sizeof(float4), ctx->stream), "clear");
     AGB_CUDA(cudaMemsetAsync(ctx->accSum.ptr, 0, n * sizeof(float4), ctx->stream), "clear");
@@ -538,7 +574,7 @@ AGB_API agb_status agb_context_memory(agb_context* ctx, uint64_t* bytes)
         ctx->matTex.bytes + ctx->instances.bytes + ctx->tlasNodes.bytes + ctx->tlasOrder.bytes + ctx->traceInst.bytes +
         ctx->layers.bytes + ctx->alias.bytes + ctx->pathState.bytes + ctx->queues.bytes +
         ctx->counters.bytes + ctx->accMean.bytes + ctx->accSum.bytes + ctx->accComp.bytes +
-        ctx->lastSample.bytes + ctx->accMoments.bytes + ctx->aovDepth.bytes + ctx->aovNormal.bytes +
+        ctx->lastSample.bytes + ctx->accMoments.bytes + ctx->post32.bytes + ctx->post8.bytes + ctx->aovDepth.bytes + ctx->aovNormal.bytes +
         ctx->aovAlbedo.bytes + ctx->aovMotion.bytes + ctx->taaHistory[0].bytes + ctx->taaHistory[1].bytes +
         uint64_t(ctx->envScratch.capacity) * 44 + ctx->stats.bytes;
     for (auto& g : ctx->geometries)
@@ -626,16 +662,21 @@ AGB_API agb_status agb_geometry_create(agb_context* ctx, const float* positions,
                 g->bounds[k]     = std::min(g->bounds[k], x);
                 g->bounds[3 + k] = std::max(g->bounds[3 + k], x);
             }
-        st = upload(ctx, g->positions, positions, size_t(vertex_count) * 3 * sizeof(float), "upload positions");
+        const size_t v3 = size_t(vertex_count) * 3 * sizeof(float), v2 = size_t(vertex_count) * 2 * sizeof(float);
+        AGB_CUDA(ensureTogether(g->arrays,
+                     { { &g->positions, v3 }, { &g->normals, normals ? v3 : 0 }, { &g->texcoords, texcoords ? v2 : 0 },
+                         { &g->indices, idx.size() * sizeof(uint32_t) }, { &g->tris, size_t(ntri) * 3 * sizeof(float4) },
+                         { &g->verts, size_t(vertex_count) * 2 * sizeof(float4) } }),
+            "allocate geometry");
+        st = upload(ctx, g->positions, positions, v3, "upload positions");
         if (!st && normals)
-            st = upload(ctx, g->normals, normals, size_t(vertex_count) * 3 * sizeof(float), "upload normals");
+            st = upload(ctx, g->normals, normals, v3, "upload normals");
         if (!st && texcoords)
-            st = upload(ctx, g->texcoords, texcoords, size_t(vertex_count) * 2 * sizeof(float), "upload texcoords");
+            st = upload(ctx, g->texcoords, texcoords, v2, "upload texcoords");
         if (!st)
             st = upload(ctx, g->indices, idx.data(), idx.size() * sizeof(uint32_t), "upload indices");
         if (st)
             return st;
-        AGB_CUDA(g->tris.ensure(size_t(ntri) * 3 * sizeof(float4)), "allocate triangles");
         GpuBvhScratch& s = ctx->bvhScratch;
         size_t capNodes  = std::max<size_t>(1, ntri);
         if (s.nodesBytes < capNodes * sizeof(BNode))
@@ -687,7 +728,6 @@ AGB_API agb_status agb_geometry_create(agb_context* ctx, const float* positions,
                 "copy BVH");
             AGB_CUDA(cudaStreamSynchronize(ctx->stream), "upload geometry");
         }
-        AGB_CUDA(g->verts.ensure(size_t(vertex_count) * 2 * sizeof(float4)), "allocate vertex records");
         AGB_CUDA(launchVertexRecords(g->positions.as<float>(), normals ? g->normals.as<float>() : nullptr,
                      texcoords ? g->texcoords.as<float>() : nullptr, vertex_count, g->verts.as<float4>(), ctx->stream),
             "build vertex records");
@@ -1387,6 +1427,9 @@ AGB_API agb_status agb_render(agb_context* ctx, const agb_render_options* opt,
         spw = uint32_t(std::max<uint64_t>(1, opt->max_paths_in_flight / pixels));
         spw = std::min(spw, std::max(1u, sample_count));
     }
+    else if (!opt->max_paths_in_flight && uint64_t(std::max(1u, sample_count)) * pixels <= ctx->pathCapacity &&
+        ctx->pathCapacity * (kPathStateBytes + kPathQueueBytes) <= AGB_WAVE_DEFAULT_BYTES)
+        spw = std::max(1u, sample_count); // one wave in the buffers at hand: no need to ask for free memory
     else
     {
         // The call's samples in as few waves as fit, split evenly.  Default: wave buffers of at
@@ -2167,7 +2210,7 @@ AGB_API agb_status agb_post_process(agb_context* ctx, int32_t mode, const float 
     if (st)
         return st;
     size_t pixels = size_t(ctx->accW) * ctx->accH;
-    DevBuf o32, o8;
+    DevBuf &o32 = ctx->post32, &o8 = ctx->post8;
     AGB_CUDA(o32.ensure(pixels * sizeof(float4)), "allocate post output");
     AGB_CUDA(o8.ensure(pixels * sizeof(uchar4)), "allocate post output");
     if (mode == AGB_POST_SOURCE_TEMPORAL && (ctx->taaLast < 0 || ctx->taaW != ctx->accW || ctx->taaH != ctx->accH))
@@ -2313,9 +2356,8 @@ AGB_API agb_status agb_tc_gemm_bf16(const uint16_t* a, const uint16_t* b, float*
         return fail(AGB_ERR_INVALID_ARG, "agb_tc_gemm_bf16: pointers must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     AGB_CUDA(launchTcGemm(a, b, d, m, n, k, st), "agb_tc_gemm_bf16");
-    AGB_CUDA(cudaStreamSynchronize(st), "agb_tc_gemm_bf16");
     int flag = 0;
-    AGB_CUDA(takeTcError(&flag), "agb_tc_gemm_bf16");
+    AGB_CUDA(takeTcError(&flag, st), "agb_tc_gemm_bf16");
     if (flag)
         return fail(AGB_ERR_TIMEOUT, "agb_tc_gemm_bf16: tensor-core completion wait timed out");
     return AGB_OK;
@@ -2346,9 +2388,8 @@ static agb_status convCommon(const char* what, const uint16_t* in0, const uint16
         up0 ? 1 : 0, relu ? 1 : 0 };
     c.pool = pool;
     AGB_CUDA(launchConv3x3(c, st), what);
-    AGB_CUDA(cudaStreamSynchronize(st), what);
     int flag = 0;
-    AGB_CUDA(takeTcError(&flag), what);
+    AGB_CUDA(takeTcError(&flag, st), what);
     if (flag)
         return fail(AGB_ERR_TIMEOUT, std::string(what) + ": tensor-core completion wait timed out");
     return AGB_OK;
@@ -2392,9 +2433,8 @@ AGB_API agb_status agb_conv3x3_wgrad_bf16(const uint16_t* in0, const uint16_t* i
     ConvLaunch c{ in0, c1 > 0 ? in1 : nullptr, nullptr, nullptr, nullptr, nullptr, batch, height, width, c0, c1, cout,
         up0 ? 1 : 0, 0 };
     AGB_CUDA(launchConvWgrad(c, dy, dw, sms, st), "agb_conv3x3_wgrad_bf16");
-    AGB_CUDA(cudaStreamSynchronize(st), "agb_conv3x3_wgrad_bf16");
     int flag = 0;
-    AGB_CUDA(takeTcError(&flag), "agb_conv3x3_wgrad_bf16");
+    AGB_CUDA(takeTcError(&flag, st), "agb_conv3x3_wgrad_bf16");
     if (flag)
         return fail(AGB_ERR_TIMEOUT, "agb_conv3x3_wgrad_bf16: tensor-core completion wait timed out");
     return AGB_OK;
@@ -2435,14 +2475,6 @@ agb_status denoiserCheck(agb_denoiser* dn, int32_t B, int32_t H, int32_t W, cons
     if (int64_t(B) * H * W >= (int64_t(1) << 26))
         return fail(AGB_ERR_LIMIT, std::string(what) + ": too many pixels per batch");
     AGB_CUDA(cudaSetDevice(dn->device), "cudaSetDevice");
-    return AGB_OK;
-}
-agb_status tcStatus(const char* what)
-{
-    int flag = 0;
-    AGB_CUDA(takeTcError(&flag), what);
-    if (flag)
-        return fail(AGB_ERR_TIMEOUT, std::string(what) + ": tensor-core completion wait timed out");
     return AGB_OK;
 }
 } // namespace
@@ -2553,12 +2585,14 @@ AGB_API agb_status agb_denoiser_train_step(agb_denoiser* dn, const uint16_t* fea
     AGB_CUDA(dn->net.backward(target_rgba), "agb_denoiser_train_step");
     if (update)
         AGB_CUDA(dn->net.adam(learning_rate), "agb_denoiser_train_step");
-    float l = 0.f;
-    AGB_CUDA(cudaMemcpyAsync(&l, dn->net.lossDevice(), 4, cudaMemcpyDeviceToHost, dn->stream), "read loss");
-    AGB_CUDA(cudaStreamSynchronize(dn->stream), "agb_denoiser_train_step");
+    bool timedOut = false;
+    float l       = 0.f;
+    AGB_CUDA(dn->net.finishStep(&l, &timedOut), "agb_denoiser_train_step");
     if (loss)
         *loss = l;
-    return tcStatus("agb_denoiser_train_step");
+    if (timedOut)
+        return fail(AGB_ERR_TIMEOUT, "agb_denoiser_train_step: tensor-core completion wait timed out");
+    return AGB_OK;
 }
 
 AGB_API agb_status agb_denoiser_features(agb_context* ctx, uint16_t* out_features)

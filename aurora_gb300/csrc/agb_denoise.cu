@@ -135,13 +135,17 @@ cudaError_t launchTcGemm(const uint16_t* A, const uint16_t* B, float* D, int M, 
     return cudaGetLastError();
 }
 
-cudaError_t takeTcError(int* flag)
+cudaError_t takeTcError(int* flag, cudaStream_t st)
 {
-    cudaError_t e = cudaMemcpyFromSymbol(flag, g_tcError, sizeof(int));
+    int* dev      = nullptr;
+    cudaError_t e = tcErrorFlag(&dev);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(flag, dev, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(st);
     if (e != cudaSuccess || *flag == 0)
         return e;
-    int zero = 0;
-    return cudaMemcpyToSymbol(g_tcError, &zero, sizeof(int));
+    return cudaMemset(dev, 0, sizeof(int));
 }
 
 cudaError_t tcErrorFlag(int** flag) { return cudaGetSymbolAddress(reinterpret_cast<void**>(flag), g_tcError); }

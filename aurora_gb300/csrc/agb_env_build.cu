@@ -14,6 +14,8 @@
 //   1 + S_{j+1} - D_after and aliases heavy j + 1.
 // This is the greedy sweep of Vose's method with the state expressed through prefix sums, so each
 // entry is independent: one binary search per texel.  All prefix sums are FP64.
+#include <type_traits>
+
 #include "agb_kernels.h"
 
 namespace agb
@@ -665,15 +667,7 @@ __global__ void k_ref_pack(const uint32_t* indexMap, const uint32_t* posAlias, c
 
 void freeEnvScratch(EnvBuildScratch& s)
 {
-    cudaFree(s.weights);
-    cudaFree(s.scanA);
-    cudaFree(s.ranks);
-    cudaFree(s.heavyIdx);
-    cudaFree(s.heavyIncl);
-    cudaFree(s.lightIncl);
-    cudaFree(s.blockSums);
-    cudaFree(s.blockCounts);
-    cudaFree(s.rowSA);
+    cudaFree(s.weights); // the first array of the one allocation that holds all
     s = EnvBuildScratch();
 }
 
@@ -684,28 +678,38 @@ cudaError_t buildEnvAlias(const float4* rgba, uint32_t width, uint32_t height, i
     const float* rowSolidAngle, agb_alias_entry* out, double* integralFP64Out,
     float* integralShadingOut, EnvBuildScratch& s, cudaStream_t st)
 {
-    uint32_t n     = width * height;
-    uint32_t tiles = (n + kScanTile - 1) / kScanTile;
+    uint32_t n = width * height;
     if (s.capacity < n || s.rows < height)
     {
         freeEnvScratch(s);
-        size_t tileCap = envScratchTileDoubles(n);
-        cudaError_t e  = cudaSuccess;
-        if ((e = cudaMalloc(&s.weights, sizeof(double) * n)) != cudaSuccess ||
-            (e = cudaMalloc(&s.scanA, sizeof(double) * n)) != cudaSuccess ||
-            (e = cudaMalloc(&s.ranks, sizeof(uint32_t) * n * 2)) != cudaSuccess ||
-            (e = cudaMalloc(&s.heavyIdx, sizeof(uint32_t) * n)) != cudaSuccess ||
-            (e = cudaMalloc(&s.heavyIncl, sizeof(double) * n)) != cudaSuccess ||
-            (e = cudaMalloc(&s.lightIncl, sizeof(double) * n)) != cudaSuccess ||
-            (e = cudaMalloc(&s.blockSums, sizeof(double) * tileCap)) != cudaSuccess ||
-            (e = cudaMalloc(&s.blockCounts, sizeof(uint32_t) * envScratchTileCounts(n))) != cudaSuccess ||
-            (e = cudaMalloc(&s.rowSA, sizeof(float) * height + 16)) != cudaSuccess)
-        {
-            freeEnvScratch(s);
+        // One allocation, carved in 256-byte steps; the first array's pointer owns it.
+        char* base  = nullptr;
+        size_t size = 0;
+        EnvBuildScratch t;
+        auto take = [&](auto*& p, size_t count) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + size);
+            size += (count * sizeof(*p) + 255) & ~size_t(255);
+        };
+        auto carve = [&]() {
+            size = 0;
+            take(t.weights, n);
+            take(t.scanA, n);
+            take(t.ranks, size_t(n) * 2);
+            take(t.heavyIdx, n);
+            take(t.heavyIncl, n);
+            take(t.lightIncl, n);
+            take(t.blockSums, envScratchTileDoubles(n));
+            take(t.blockCounts, envScratchTileCounts(n));
+            take(t.rowSA, size_t(height) + 4);
+        };
+        carve();
+        const cudaError_t e = cudaMalloc(&base, size);
+        if (e != cudaSuccess)
             return e;
-        }
-        s.capacity = n;
-        s.rows     = height;
+        carve();
+        t.capacity = n;
+        t.rows     = height;
+        s          = t;
     }
     return launchEnvAliasBuild(rgba, width, height, layout, rowSolidAngle, out, integralFP64Out,
         integralShadingOut, s, st);

@@ -216,8 +216,9 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
 // agb_denoise.cu
 
 cudaError_t launchTcGemm(const uint16_t* A, const uint16_t* B, float* D, int M, int N, int K, cudaStream_t st);
-// Reads and clears the tensor-core kernels' timeout flag (1 = a bounded wait ran out).
-cudaError_t takeTcError(int* flag);
+// Waits for the stream, then reads and clears the tensor-core kernels' timeout flag (1 = a bounded wait ran
+// out); the copy of the flag follows the kernels on the stream, so the caller waits once.
+cudaError_t takeTcError(int* flag, cudaStream_t st);
 // Device address of that flag on the current device (kernels in other translation units set it).
 cudaError_t tcErrorFlag(int** flag);
 
@@ -242,10 +243,11 @@ public:
     // After forward(training): L1 loss against target RGBA (FP32) and all parameter gradients.
     cudaError_t backward(const float* target);
     cudaError_t adam(float lr);
+    // Waits for the step and reads its loss and whether a tensor-core wait ran out (the flag is then cleared).
+    cudaError_t finishStep(float* loss, bool* timedOut);
     cudaError_t setParams(const float* host);
     const float* params() const { return params_; }
     const float* grads() const { return grads_; }
-    const float* lossDevice() const { return loss_; }
     size_t nParams() const { return nParams_; }
     static double flopsPerPixel(bool training);
     void release();
@@ -287,7 +289,14 @@ private:
     };
     std::vector<Graph> graphs_; // most recently used last
     Graph pending_{};           // buffers seen once, captured when seen again
-    int* flagHost_ = nullptr;   // pinned copy of the tensor-core timeout flag
+    // Pinned copies of the tensor-core timeout flag and of a step's loss.
+    struct HostWords
+    {
+        int flag;
+        float loss;
+    };
+    HostWords* host_ = nullptr;
+    cudaError_t ensureHost();
 };
 cudaError_t launchDenoiseFeatures(const float4* mean, const float2* moments, float samples, const float4* albedo,
     const float4* normal, const float* depth, float skyZ, long P, uint16_t* out, cudaStream_t st);
@@ -295,18 +304,14 @@ cudaError_t launchDenoiseFeatures(const float4* mean, const float2* moments, flo
 // agb_bvh_gpu.cu: binned-SAH BLAS build on the GPU.
 struct GpuBvhScratch
 {
-    float* boxes      = nullptr;
-    size_t boxesBytes = 0;
-    uint32_t* order   = nullptr;
-    size_t orderBytes = 0;
-    uint32_t* scratch = nullptr;
-    size_t scratchBytes = 0;
-    void* tasksA      = nullptr;
-    size_t tasksABytes = 0;
-    void* tasksB      = nullptr;
-    size_t tasksBBytes = 0;
-    void* counters    = nullptr;
-    size_t countersBytes = 0;
+    void* arrays       = nullptr; // one allocation that holds the six below
+    size_t arraysBytes = 0;
+    float* boxes       = nullptr;
+    uint32_t* order    = nullptr;
+    uint32_t* scratch  = nullptr;
+    void* big          = nullptr; // the large nodes' arrays
+    void* subtrees     = nullptr; // the subtree list
+    void* counters     = nullptr;
     BNode* nodes      = nullptr;
     size_t nodesBytes = 0;
 };

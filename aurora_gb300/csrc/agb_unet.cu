@@ -282,9 +282,9 @@ void UnetDenoiser::dropGraphs()
 void UnetDenoiser::release()
 {
     dropGraphs();
-    if (flagHost_)
-        cudaFreeHost(flagHost_);
-    flagHost_ = nullptr;
+    if (host_)
+        cudaFreeHost(host_);
+    host_ = nullptr;
     for (void* p : allocs_)
         cudaFree(p);
     allocs_.clear();
@@ -463,34 +463,52 @@ cudaError_t UnetDenoiser::forward(const uint16_t* x, int B, int H, int W, bool t
     return cudaSuccess;
 }
 
+cudaError_t UnetDenoiser::ensureHost()
+{
+    if (host_)
+        return cudaSuccess;
+    const cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&host_), sizeof(HostWords));
+    if (e == cudaSuccess)
+        *host_ = HostWords{ 0, 0.f };
+    return e;
+}
+
 bool UnetDenoiser::inferTimedOut()
 {
-    if (!flagHost_ || *flagHost_ == 0)
+    if (!host_ || host_->flag == 0)
         return false;
     int flag = 0;
-    takeTcError(&flag);
-    *flagHost_ = 0;
+    takeTcError(&flag, stream_);
+    host_->flag = 0;
     return true;
+}
+
+cudaError_t UnetDenoiser::finishStep(float* loss, bool* timedOut)
+{
+    int* flagDev  = nullptr;
+    cudaError_t e = ensureHost();
+    if (e != cudaSuccess || (e = tcErrorFlag(&flagDev)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&host_->loss, loss_, sizeof(float), cudaMemcpyDeviceToHost, stream_)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&host_->flag, flagDev, sizeof(int), cudaMemcpyDeviceToHost, stream_)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(stream_)) != cudaSuccess)
+        return e;
+    *loss     = host_->loss;
+    *timedOut = inferTimedOut();
+    return cudaSuccess;
 }
 
 cudaError_t UnetDenoiser::infer(const uint16_t* x, int B, int H, int W, float* rgba)
 {
     cudaError_t e = ensureShape(B, H, W, false);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess || (e = ensureHost()) != cudaSuccess)
         return e;
-    if (!flagHost_)
-    {
-        if ((e = cudaMallocHost(reinterpret_cast<void**>(&flagHost_), sizeof(int))) != cudaSuccess)
-            return e;
-        *flagHost_ = 0;
-    }
     int* flagDev = nullptr;
     if ((e = tcErrorFlag(&flagDev)) != cudaSuccess)
         return e;
     e = inferLaunch(x, B, H, W, rgba);
     if (e != cudaSuccess)
         return e;
-    return cudaMemcpyAsync(flagHost_, flagDev, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+    return cudaMemcpyAsync(&host_->flag, flagDev, sizeof(int), cudaMemcpyDeviceToHost, stream_);
 }
 
 cudaError_t UnetDenoiser::inferLaunch(const uint16_t* x, int B, int H, int W, float* rgba)
