@@ -24,8 +24,9 @@
 //            one 1D bulk copy, into a ring of `stages` shared-memory stages (full / empty
 //            mbarriers);
 //   warp 1   MMA issuer: per stage 2 R x 9 tcgen05.mma (M = 128, N, K = 16) into the tile's
-//            accumulators in TMEM, double-buffered (2 x 256 columns) so that the epilogue of one
-//            tile overlaps the MMAs of the next;
+//            accumulators in TMEM, double-buffered (2 x 256 columns; four rows of 64 channels take
+//            all 512, freed two rows at a time) so that the epilogue of one tile overlaps the MMAs
+//            of the next;
 //   warps 2-9 epilogue: tcgen05.ld of the accumulators, + bias, optional ReLU, BF16 (and / or FP32)
 //            NHWC stores, and optionally the 2x2 average pool of the BF16 outputs (the encoder's
 //            downsampling, exactly as a separate pool over the stored values would compute it).
@@ -130,8 +131,10 @@ __device__ __forceinline__ float bfv(uint16_t b) { return __uint_as_float(uint32
 
 // Output rows per tile for N output channels: as many as one TMEM buffer of 256 columns holds
 // (2 R N), at most 4 (six rows for 16 channels measured slower: 77 against 66 us for the output
-// layer at 1920x1080).
+// layer at 1920x1080); see launchConv3x3 for the four-row tiles of 64 channels.
 __host__ __device__ constexpr int tileRows(int n) { return n >= 64 ? 2 : 4; }
+// Accumulator buffers: two of 256 columns, or one that takes the whole TMEM.
+__host__ __device__ constexpr int accBuffers(int n, int r) { return 2 * r * n <= int(kAccStride) ? 2 : 1; }
 
 // The MMAs of one pipeline stage (one 16-channel input group), fully unrolled.  Halo row i (input
 // row y0 - 1 + i) feeds output rows r = i - 2 .. i (those inside the tile) through the vertical taps
@@ -139,11 +142,11 @@ __host__ __device__ constexpr int tileRows(int n) { return n >= 64 ? 2 : 4; }
 // stacked (dy = 2, 1, 0), so one MMA per (halo row, parity, dx) covers every output row the halo
 // row feeds: N, 2N or 3N accumulator columns at once.  In the first group of a tile an
 // accumulator starts its sum (accumulate = 0) with the dx = 0 MMA of halo row r, split off as an
-// MMA of its own.
-template <int N, bool UP>
-__device__ __forceinline__ void issueStage(uint32_t aAddr, uint32_t bAddr, uint32_t dBase, bool first)
+// MMA of its own.  rowsFree(r) is called before the first MMA that writes output rows r and r + 1.
+template <int N, int R, bool UP, class RowsFree>
+__device__ __forceinline__ void issueStage(uint32_t aAddr, uint32_t bAddr, uint32_t dBase, bool first,
+    const RowsFree& rowsFree)
 {
-    constexpr int R = tileRows(N);
     // K-major, 32-byte swizzle: entries of 32 bytes (16 channels), 8-entry atoms 256 bytes apart.
     const uint64_t aDesc0 = tc::smemDescSw32(aAddr, 256);
     const uint64_t bDesc0 = tc::smemDesc(bAddr, tc::kSliceLbo, tc::kSliceSbo);
@@ -153,6 +156,8 @@ __device__ __forceinline__ void issueStage(uint32_t aAddr, uint32_t bAddr, uint3
         const int rLo   = i - 2 > 0 ? i - 2 : 0;
         const int rHi   = i < R - 1 ? i : R - 1;
         const int count = rHi - rLo + 1;
+        if (i % 2 == 0 && i < R)
+            rowsFree(i);
 #pragma unroll
         for (int par = 0; par < 2; par++)
 #pragma unroll
@@ -247,13 +252,16 @@ __device__ __forceinline__ void warpAddChannels(float (&v)[16], float* dst, int 
         atomicAdd(dst + (lane >> 1), v[0]);
 }
 
-template <int N, bool SPLIT>
+template <int N, int R, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_constant__ CUtensorMap tm0,
     const __grid_constant__ CUtensorMap tm1, const ConvTmaArgs a)
 {
-    constexpr int R = tileRows(N);
+    // Two buffers are freed as wholes; one is freed two rows at a time, so that the next tile's MMAs of its
+    // first rows overlap the epilogue of the last ones.
+    constexpr int kBuffers = accBuffers(N, R);
+    constexpr int kFrees   = kBuffers == 2 ? 1 : R / 2; // parts of a buffer that are freed apart
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], accFull[2], accEmpty[2], drain;
+    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], accFull[kBuffers], accEmpty[kBuffers * kFrees], drain;
     __shared__ uint32_t tmemBase;
     __shared__ float biasGrad[SPLIT ? kMaxGradChannels : 1]; // this CTA's share of db0
     const int tid  = threadIdx.x;
@@ -273,11 +281,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
             tc::mbarInit(&full[s], 1);
             tc::mbarInit(&empty[s], 1);
         }
-        for (int i = 0; i < 2; i++)
-        {
+        for (int i = 0; i < kBuffers; i++)
             tc::mbarInit(&accFull[i], 1);
+        for (int i = 0; i < kBuffers * kFrees; i++)
             tc::mbarInit(&accEmpty[i], 8);
-        }
         tc::mbarInit(&drain, 1);
         tc::fenceMbarInit();
     }
@@ -356,14 +363,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
             int k       = 0;
             for (int t = blockIdx.x; t < a.numTiles && ok; t += gridDim.x, k++)
             {
-                const int buf      = k & 1;
-                const uint32_t aph = uint32_t(k >> 1) & 1u;
-                if (!tc::mbarWait(&accEmpty[buf], aph ^ 1u))
+                const int buf      = k % kBuffers;
+                const uint32_t aph = uint32_t(k / kBuffers) & 1u;
+                if (kFrees == 1)
                 {
-                    ok = false;
-                    break;
+                    if (!tc::mbarWait(&accEmpty[buf], aph ^ 1u))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    tc::fenceAfterSync();
                 }
-                tc::fenceAfterSync();
+                auto rowsFree = [&](int r) {
+                    if (!tc::mbarWait(&accEmpty[r / 2], aph ^ 1u))
+                        ok = false;
+                    tc::fenceAfterSync();
+                };
+                auto rowsHeld = [](int) {};
                 const uint32_t dBase = tmem + uint32_t(buf) * kAccStride;
                 for (int g = 0; g < a.G; g++, it++)
                 {
@@ -377,10 +393,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                     tc::fenceAfterSync();
                     const uint32_t aAddr = tc::smemAddr(smem + size_t(s) * a.stageBytes);
                     const uint32_t bAddr = aAddr + a.aBytes;
-                    if (g < a.G0 && a.up0)
-                        issueStage<N, true>(aAddr, bAddr, dBase, g == 0);
+                    if constexpr (kFrees > 1)
+                    {
+                        if (g == 0)
+                        {
+                            if (a.up0)
+                                issueStage<N, R, true>(aAddr, bAddr, dBase, true, rowsFree);
+                            else
+                                issueStage<N, R, false>(aAddr, bAddr, dBase, true, rowsFree);
+                        }
+                        else if (g < a.G0 && a.up0)
+                            issueStage<N, R, true>(aAddr, bAddr, dBase, false, rowsHeld);
+                        else
+                            issueStage<N, R, false>(aAddr, bAddr, dBase, false, rowsHeld);
+                    }
+                    else if (g < a.G0 && a.up0)
+                        issueStage<N, R, true>(aAddr, bAddr, dBase, g == 0, rowsHeld);
                     else
-                        issueStage<N, false>(aAddr, bAddr, dBase, g == 0);
+                        issueStage<N, R, false>(aAddr, bAddr, dBase, g == 0, rowsHeld);
                     tc::commit(&empty[s]);
                 }
                 if (!ok)
@@ -414,8 +444,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
         for (int t = blockIdx.x; t < a.numTiles; t += gridDim.x, k++)
         {
             const Tile q       = decodeTile(a, t);
-            const int buf      = k & 1;
-            const uint32_t aph = uint32_t(k >> 1) & 1u;
+            const int buf      = k % kBuffers;
+            const uint32_t aph = uint32_t(k / kBuffers) & 1u;
             if (!leaderWait(&accFull[buf], aph, lane))
             {
                 ok = false;
@@ -430,6 +460,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
             {
                 const int r  = (item / chunks) * step;
                 const int c0 = (item % chunks) * 16;
+                if (kFrees > 1 && item >= chunks && item - 2 < (item / chunks) * chunks)
+                {
+                    // This warp's first item of a new row pair: it is done with the one before.
+                    tc::fenceBeforeSync();
+                    __syncwarp();
+                    if (lane == 0)
+                        tc::mbarArrive(&accEmpty[item / chunks - 1]);
+                }
                 // All accumulators of the item (2 or 4) in flight before one wait.
                 uint32_t v[4][16];
                 // Accumulator (row r, parity p) at columns (p R + r) N.
@@ -575,7 +613,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
             tc::fenceBeforeSync();
             __syncwarp();
             if (lane == 0)
-                tc::mbarArrive(&accEmpty[buf]);
+                tc::mbarArrive(&accEmpty[buf * kFrees + kFrees - 1]);
         }
     }
     tc::fenceBeforeSync();
@@ -966,12 +1004,24 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     a.B = c.B, a.H = c.H, a.W = c.W, a.Cout = c.Cout, a.up0 = c.up0, a.relu = c.relu;
     a.N      = convTileChannels(c.Cout);
     a.nTiles = c.Cout / a.N;
-    a.R      = tileRows(a.N);
     a.G         = (c.C0 + c.C1) / 16;
     a.G0        = c.C0 / 16;
     a.tilesX    = (c.W / 2 + 127) / 128;
+    int dev     = 0;
+    if (cudaError_t ed = cudaGetDevice(&dev); ed != cudaSuccess)
+        return ed;
+    const int sms    = smCountOf(dev);
+    auto tilesOf     = [&](int rows) { return long(c.B) * ((c.H + rows - 1) / rows) * a.tilesX * a.nTiles; };
+    a.R              = tileRows(a.N);
+    // Four rows of 64 channels take the whole TMEM, so a tile's epilogue holds up the next tile's MMAs in part;
+    // but halo rows, weights and MMA operands are read for twice the outputs (414 cycles of MMAs for a 16-channel
+    // group instead of 2 x 222).  Worth it from 128 input channels on: 960x540, 128 up + 64 to 64 channels
+    // 111.4 us with two rows, 98.7 with four; 1920x1080 inference 948 us with two rows everywhere, 910 with
+    // four from 128 input channels, 923 with four from 64.
+    if (a.N == 64 && a.G >= 8 && (tilesOf(4) + sms - 1) / sms * 414 <= (tilesOf(2) + sms - 1) / sms * 222)
+        a.R = 4;
     a.rowBlocks = (c.H + a.R - 1) / a.R;
-    long tiles  = long(c.B) * a.rowBlocks * a.tilesX * a.nTiles;
+    long tiles  = tilesOf(a.R);
     if (tiles >= (1L << 31))
         return cudaErrorInvalidValue;
     a.numTiles   = int(tiles);
@@ -997,14 +1047,13 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     // At least half of the SM's shared memory, so that one CTA (with all 512 TMEM columns) runs
     // per SM.
     const size_t smem = std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024);
-    auto kern        = split ? (a.N == 64 ? k_conv3x3_tma<64, true> : a.N == 32 ? k_conv3x3_tma<32, true> : k_conv3x3_tma<16, true>)
-                             : (a.N == 64 ? k_conv3x3_tma<64, false> : a.N == 32 ? k_conv3x3_tma<32, false> : k_conv3x3_tma<16, false>);
+    auto kern = split ? (a.N == 64 ? (a.R == 4 ? k_conv3x3_tma<64, 4, true> : k_conv3x3_tma<64, 2, true>)
+                            : a.N == 32 ? k_conv3x3_tma<32, 4, true> : k_conv3x3_tma<16, 4, true>)
+                      : (a.N == 64 ? (a.R == 4 ? k_conv3x3_tma<64, 4, false> : k_conv3x3_tma<64, 2, false>)
+                            : a.N == 32 ? k_conv3x3_tma<32, 4, false> : k_conv3x3_tma<16, 4, false>);
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
         return e;
-    int dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess)
-        return e;
-    const int grid = int(std::min<long>(tiles, smCountOf(dev)));
+    const int grid = int(std::min<long>(tiles, sms));
     return launchOverlapped(kern, unsigned(grid), kThreads, smem, st, m0, m1, a);
 }
 
