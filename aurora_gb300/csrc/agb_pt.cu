@@ -197,22 +197,28 @@ struct OcclusionWriter
 
 // Transparent shadows (is_force_opaque_shadows_enabled = 0): the any-hit shader of
 // HitShaderEntryPoints.slang:490-552 multiplies the ray's visibility by 1 - opacity at every
-// surface it crosses and ends the ray once it is black.  Here the hits are taken nearest first,
-// each by a closest-hit traversal from just beyond the previous one, so the product has one
-// order; at most kMaxShadowHits are taken.
+// surface it crosses and ends the ray once it is black.  Here a blocking surface ends the ray wherever it is
+// found; the hits of a ray that meets none are taken nearest first, each by a closest-hit traversal
+// from just beyond the previous one, so the product has one order; at most kMaxShadowHits are taken.
 constexpr int kMaxShadowHits = 4096;
+
+// Whether an instance blocks shadow rays completely: an opaque material without an opacity texture.
+AGB_D bool shadowOpaque(const DevScene& s, const DevInstance& in)
+{
+    const agb_material& b = s.materials[in.material];
+    bool hasOpacityImage  = s.matTex && b.has_opacity_image && s.matTex[in.material].image[AGB_TEX_OPACITY] >= 0;
+    // A node-graph program may drive the opacity: such a material is never taken as opaque here.
+    bool hasGraph = s.matGraph && s.matGraph[in.material].y > 0;
+    return b.opacity[0] == 1.f && b.opacity[1] == 1.f && b.opacity[2] == 1.f && !hasOpacityImage && !hasGraph &&
+        b.transmission == 0.f;
+}
 
 // Opacity the any-hit shader takes from a hit: the instance's material opacity x (1 -
 // transmission x transmission colour), 1 for an opaque material without an opacity texture.
 AGB_DN v3 shadowOpacity(const DevScene& s, const RayHit& h)
 {
     const DevInstance& in = s.instances[h.inst];
-    const agb_material& b = s.materials[in.material];
-    bool hasOpacityImage  = s.matTex && b.has_opacity_image && s.matTex[in.material].image[AGB_TEX_OPACITY] >= 0;
-    // A node-graph program may drive the opacity: such a material is never taken as opaque here.
-    bool hasGraph = s.matGraph && s.matGraph[in.material].y > 0;
-    if (b.opacity[0] == 1.f && b.opacity[1] == 1.f && b.opacity[2] == 1.f && !hasOpacityImage && !hasGraph &&
-        b.transmission == 0.f)
+    if (shadowOpaque(s, in))
         return splat(1.f);
     Shading sh = computeShading(s, in, uint32_t(h.prim), h.u, h.v);
     v3 mn      = sh.N;
@@ -245,6 +251,10 @@ struct TransparentShadowWriter
     const uint32_t* tag;
     float4* vis;
     float4* pendSlot;
+    // A blocking surface makes the product zero wherever it lies along the ray, so the first one found
+    // ends the search, as for opaque shadow rays (961x541, 4 samples of the layered scene type: 1.40 -> 1.32 ms
+    // of the launches that trace both kinds of ray).
+    AGB_D bool endsAt(const DevScene& s, int32_t inst) const { return shadowOpaque(s, s.instances[inst]); }
     // Returns false (trace on from the new tmin) while the ray is not blocked.
     AGB_D bool operator()(const DevScene& s, uint32_t i, bool hit, const RayHit& h, float& tmin) const
     {

@@ -244,7 +244,8 @@ constexpr int kNodeSteps = 2;
 
 // A Writer whose kRestart is true is called as write(scene, ray, hit?, hit, tmin) and returns
 // false to trace the same ray again from the tmin it sets (transparent shadows walk the hits
-// along the ray this way); other writers are called as write(ray, hit?, hit) and end the ray.
+// along the ray this way); endsAt(scene, instance) says that a hit on the instance ends the ray wherever
+// it lies, so the search stops there.  Other writers are called as write(ray, hit?, hit) and end the ray.
 template <class W, class = void>
 struct WriterRestarts
 {
@@ -439,7 +440,10 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
                     hit.inst = inst;
                     hit.prim = prim;
                 }
-                if (kAnyHit)
+                bool ends = kAnyHit;
+                if constexpr (WriterRestarts<Writer>::value)
+                    ends = write.endsAt(s, inst);
+                if (ends)
                 {
                     ref = kDone, sp = 0;
                     cur = end = 0;
