@@ -640,10 +640,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
 // MMA covers all nine taps' rows for its horizontal tap - otherwise a work item takes one dy and
 // 128 input channels.  Accumulators: the three horizontal taps x N columns in TMEM, summed over
 // the item's units, then added to dW with vector reductions (red.global.add.v4.f32).
-constexpr uint32_t kWgEntriesA = 66;   // 64 pairs + offsets 0..2
-constexpr uint32_t kWgEntriesB = 64;
-constexpr uint32_t kWgSlotA    = 2304; // 66 x 32 bytes rounded up to the 256-byte swizzle atom
-constexpr uint32_t kWgSlotB    = 2048; // 64 x 32 bytes
+constexpr uint32_t kWgSlotA    = 2304; // 72 entries of 32 bytes: 1 x 66, 2 x 34 or 4 x 18 (64 pairs, offsets 0..2)
+constexpr uint32_t kWgSlotB    = 2048; // 64 entries
 constexpr int kWgThreads       = 192;  // producer, MMA issuer, 4 epilogue warps
 constexpr int kWgMaxStages     = 6;
 
@@ -655,6 +653,9 @@ struct WgradTmaArgs
     int Gci;             // 16-channel groups of X per tap in an item
     int ciTiles, coTiles, N, splits;
     int unitsX, numUnits, unitsPerItem, numItems;
+    int rows, rowBlocks; // image rows of a unit, units down an image
+    int steps;           // K steps (of 16 pairs) of a unit's row
+    int entriesA;        // of a staged row of X: 16 steps + 2
     uint32_t stageBytes, aBytes;
     int stages;
     int* error;
@@ -720,8 +721,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
             bool issued[kWgMaxStages];
             for (int s = 0; s < S; s++)
                 issued[s] = false;
-            const uint32_t bytesA = uint32_t(a.T * a.Gci) * 2u * kWgEntriesA * 32u;
-            const uint32_t bytesB = uint32_t(N / 16) * 2u * kWgEntriesB * 32u;
+            const uint32_t bytesA = uint32_t(a.T * a.Gci) * 2u * uint32_t(a.rows * a.entriesA) * 32u;
+            const uint32_t bytesB = uint32_t(N / 16) * 2u * uint32_t(a.rows * a.steps) * 16u * 32u;
             uint32_t it = 0;
             for (int u = u0; u < u1; u++, it++)
             {
@@ -734,8 +735,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
                 }
                 const int xs = u % a.unitsX;
                 const int r  = u / a.unitsX;
-                const int y  = r % a.H;
-                const int b  = r / a.H;
+                const int y  = (r % a.rowBlocks) * a.rows;
+                const int b  = r / a.rowBlocks;
                 const int j0 = xs * 64;
                 uint8_t* A   = smem + size_t(s) * a.stageBytes;
                 uint8_t* Bm  = A + a.aBytes;
@@ -780,9 +781,18 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
         {
             // MN-major A and B (bits 15, 16), M = 128, N.
             const uint32_t idesc = tc::idescBf16(128, N) | (1u << 15) | (1u << 16);
-            uint32_t it          = 0;
+            // K step k of a unit: its row's staged entries, 16 pairs on (in 16-byte units).
+            uint32_t stepA[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                stepA[k] = uint32_t((k / a.steps) * a.entriesA + (k % a.steps) * 16) * 2u;
+            uint32_t it = 0;
             for (int u = u0; u < u1; u++, it++)
             {
+                // Steps within the image: pairs and rows beyond it are staged as zeros.
+                const int pairs  = a.W / 2 - (u % a.unitsX) * 64;
+                const int across = min(a.steps, (pairs + 15) / 16);
+                const int steps  = across * min(a.rows, a.H - (u / a.unitsX) % a.rowBlocks * a.rows);
                 const bool first   = u == u0 || u == mid;
                 const uint32_t acc = tmem + (u < mid ? 0u : 3u * N);
                 const int s       = int(it % uint32_t(S));
@@ -810,9 +820,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
                         const uint64_t bd    = bDesc0 + ((uint32_t(par) * (N / 16) * kWgSlotB) >> 4);
 #pragma unroll
                         for (int ks = 0; ks < 4; ks++)
-                            tc::mma(acc + uint32_t(dx * N), ad + ((uint32_t(ks) * 16u * 32u) >> 4),
-                                bd + ((uint32_t(ks) * 16u * 32u) >> 4), idesc,
-                                (first && par == 0 && ks == 0) ? 0u : 1u);
+                            if (ks < steps)
+                                tc::mma(acc + uint32_t(dx * N), ad + stepA[ks], bd + ((uint32_t(ks) * 16u * 32u) >> 4),
+                                    idesc, (first && par == 0 && ks == 0) ? 0u : 1u);
                     }
                 tc::commit(&empty[s]);
             }
@@ -895,15 +905,16 @@ PFN_cuTensorMapEncodeTiled_v12000 encodeTiled()
 }
 
 // Even / odd view of a full-resolution NHWC BF16 tensor: (C, parity, W / 2, H, B), box 16 x 1 x
-// entries, 32-byte swizzle.
-cudaError_t mapPairs(CUtensorMap* m, const uint16_t* base, int B, int H, int W, int C, int entries = kHaloEntries)
+// entries x rows, 32-byte swizzle.
+cudaError_t mapPairs(CUtensorMap* m, const uint16_t* base, int B, int H, int W, int C, int entries = kHaloEntries,
+    int rows = 1)
 {
     auto enc = encodeTiled();
     if (!enc)
         return cudaErrorNotSupported;
     cuuint64_t dims[5]    = { cuuint64_t(C), 2, cuuint64_t(W / 2), cuuint64_t(H), cuuint64_t(B) };
     cuuint64_t strides[4] = { cuuint64_t(C) * 2, cuuint64_t(C) * 4, cuuint64_t(W) * C * 2, cuuint64_t(H) * W * C * 2 };
-    cuuint32_t box[5]     = { 16, 1, cuuint32_t(entries), 1, 1 };
+    cuuint32_t box[5]     = { 16, 1, cuuint32_t(entries), cuuint32_t(rows), 1 };
     cuuint32_t es[5]      = { 1, 1, 1, 1, 1 };
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<uint16_t*>(base), dims, strides, box, es,
         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1071,8 +1082,16 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     if (c.Cout % a.N || (a.N != 16 && a.N != 32 && a.N != 48 && a.N != 64 && a.N != 96 && a.N != 128))
         return cudaErrorInvalidValue;
     a.coTiles  = c.Cout / a.N;
-    a.unitsX   = (c.W / 2 + 63) / 64;
-    a.numUnits = c.B * c.H * a.unitsX;
+    a.unitsX = (c.W / 2 + 63) / 64;
+    // Narrow images: a unit is as many rows as make 64 pairs (one row of an upsampled source, whose staged
+    // rows repeat).  Single rows leave up to three quarters of a unit's loads and MMAs to padding: the six
+    // weight gradients of 64x64 and 32x32 images in a training step on four 256x256 crops 350 us with
+    // them, 307 so (launches overlap), the step 1386 and 1364 us.
+    a.steps     = std::min(4, (c.W / 2 + 15) / 16);
+    a.rows      = c.up0 ? 1 : 4 / a.steps;
+    a.rowBlocks = (c.H + a.rows - 1) / a.rows;
+    a.entriesA  = 16 * a.steps + 2;
+    a.numUnits  = c.B * a.rowBlocks * a.unitsX;
     const int fixedItems = (a.T == 3 ? 1 : 3) * a.ciTiles * a.coTiles;
     const int sms        = smCount > 0 ? smCount : 148;
     // A CTA takes a whole SM.  Two items per SM; where the kernel sums two halves of an item apart, two at most
@@ -1098,18 +1117,18 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     if (e != cudaSuccess)
         return e;
     CUtensorMap m0, m1, md;
-    e = c.up0 ? mapRows(&m0, c.in0, c.B, c.H / 2, c.W / 2, c.C0, kWgEntriesA)
-              : mapPairs(&m0, c.in0, c.B, c.H, c.W, c.C0, kWgEntriesA);
+    e = c.up0 ? mapRows(&m0, c.in0, c.B, c.H / 2, c.W / 2, c.C0, a.entriesA)
+              : mapPairs(&m0, c.in0, c.B, c.H, c.W, c.C0, a.entriesA, a.rows);
     if (e != cudaSuccess)
         return e;
     if (c.C1 > 0)
     {
-        if ((e = mapPairs(&m1, c.in1, c.B, c.H, c.W, c.C1, kWgEntriesA)) != cudaSuccess)
+        if ((e = mapPairs(&m1, c.in1, c.B, c.H, c.W, c.C1, a.entriesA, a.rows)) != cudaSuccess)
             return e;
     }
     else
         m1 = m0;
-    if ((e = mapPairs(&md, dy, c.B, c.H, c.W, c.Cout, kWgEntriesB)) != cudaSuccess)
+    if ((e = mapPairs(&md, dy, c.B, c.H, c.W, c.Cout, 16 * a.steps, a.rows)) != cudaSuccess)
         return e;
     // The stages, or the epilogue's rows (three times 128) in their place.
     const size_t smem = std::max<size_t>(std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024),
