@@ -2,7 +2,7 @@
 // implicit GEMM fed by TMA tensor copies.
 //
 // Work unit (tile): R consecutive output rows x 256 consecutive output pixels x N output channels
-// of one image.  The 256 pixels are split by parity into two MMA tiles of 128 rows: even pixels
+// of one image, or of several narrow images side by side.  The 256 pixels are split by parity into two MMA tiles of 128 rows: even pixels
 // x = 2j and odd pixels x = 2j + 1, j in [j0, j0 + 128).  Every input that a tap of such a tile
 // reads is then a run of 128 consecutive entries of a 130-entry "halo row" at offset 0, 1 or 2:
 //   - a full-resolution input row is staged as its even-pixel row E and its odd-pixel row O
@@ -11,7 +11,7 @@
 //   - a nearest-2x-upsampled input (the decoder's in0) is staged at its own half resolution
 //     (pixels j0 - 1 .. j0 + 128 of row (y + dy) >> 1), and the same taps read it at offsets
 //     0, 1, 1 (even) and 1, 1, 2 (odd): the upsample costs nothing and is never materialised.
-// A staged row is one TMA box (16 channels x 130 entries, 32 bytes per entry) in the K-major
+// A staged row is one TMA box (16 channels x 130 entries, fewer in a narrow image, 32 bytes per entry) in the K-major
 // 32-byte-swizzled layout: the 16-byte halves of entry i sit at 32 i and 32 i + 16, exchanged when
 // bit 7 of the address is set.  Both the TMA write and the MMA read apply the swizzle to the shared
 // memory address itself, so an A descriptor started 32 bytes per entry of offset later addresses
@@ -50,8 +50,7 @@ namespace
 
 constexpr int kHaloEntries      = 130;               // 128 MMA rows + offsets 0..2
 constexpr uint32_t kEntryBytes  = 32;                // 16 channels of one entry
-constexpr uint32_t kBoxBytes    = kHaloEntries * kEntryBytes; // one TMA box: 16 channels x 130 entries
-constexpr uint32_t kRowBytes    = 4352;              // kBoxBytes rounded up to 256 (the swizzle atom)
+constexpr uint32_t kRowBytes    = 4352;              // a box of 130 entries rounded up to 256 (the swizzle atom)
 constexpr int kThreads          = 320; // producer, MMA issuer, 8 epilogue warps
 constexpr uint32_t kAccStride   = 256;               // TMEM columns per accumulator buffer
 constexpr int kMaxStages        = 4;
@@ -77,6 +76,7 @@ struct ConvTmaArgs
     int B, H, W, Cout, up0, relu;
     int N, nTiles, R, G, G0, stages;
     int tilesX, rowBlocks, numTiles;
+    int images, pitch; // images of a tile, staged entries (and MMA rows) from one to the next
     uint32_t stageBytes, aBytes;
 };
 
@@ -93,7 +93,7 @@ __device__ __forceinline__ Tile decodeTile(const ConvTmaArgs& a, int t)
     q.j0 = (t % a.tilesX) * 128;
     t /= a.tilesX;
     q.y0 = (t % a.rowBlocks) * a.R;
-    q.b  = t / a.rowBlocks;
+    q.b  = t / a.rowBlocks * a.images;
     return q;
 }
 
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                     const int c     = (in0 ? g : g - a.G0) * 16;
                     const void* map = in0 ? static_cast<const void*>(&tm0) : static_cast<const void*>(&tm1);
                     const int rows  = up ? upRowCount(q.y0, R) : (R + 2) * 2;
-                    tc::mbarExpectTx(&full[s], wBytes + uint32_t(rows) * kBoxBytes);
+                    tc::mbarExpectTx(&full[s], wBytes + uint32_t(rows * a.images * a.pitch) * kEntryBytes);
                     tc::bulkLoad(Bw, a.wpack + (size_t(q.nt) * a.G + g) * 9 * size_t(N) * 16, wBytes, &full[s]);
                     if (up)
                     {
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
         int k              = 0;
         for (int t = blockIdx.x; t < a.numTiles; t += gridDim.x, k++)
         {
-            const Tile q       = decodeTile(a, t);
+            Tile q             = decodeTile(a, t);
             const int buf      = k % kBuffers;
             const uint32_t aph = uint32_t(k / kBuffers) & 1u;
             if (!leaderWait(&accFull[buf], aph, lane))
@@ -452,8 +452,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
                 break;
             }
             tc::fenceAfterSync();
-            const int j          = q.j0 + m;
-            const bool colOk     = j < W2;
+            const int j      = q.j0 + m % a.pitch;
+            const int image  = m / a.pitch;
+            q.b += image;
+            const bool colOk     = j < W2 && image < a.images && q.b < a.B;
             const int cb         = q.nt * N;
             const uint32_t tBase = tmem + (uint32_t(quad * 32) << 16) + uint32_t(buf) * kAccStride;
             for (int item = half; item < items; item += 2)
@@ -905,16 +907,16 @@ PFN_cuTensorMapEncodeTiled_v12000 encodeTiled()
 }
 
 // Even / odd view of a full-resolution NHWC BF16 tensor: (C, parity, W / 2, H, B), box 16 x 1 x
-// entries x rows, 32-byte swizzle.
-cudaError_t mapPairs(CUtensorMap* m, const uint16_t* base, int B, int H, int W, int C, int entries = kHaloEntries,
-    int rows = 1)
+// entries x rows x images, 32-byte swizzle.
+cudaError_t mapPairs(CUtensorMap* m, const uint16_t* base, int B, int H, int W, int C, int entries,
+    int rows, int images = 1)
 {
     auto enc = encodeTiled();
     if (!enc)
         return cudaErrorNotSupported;
     cuuint64_t dims[5]    = { cuuint64_t(C), 2, cuuint64_t(W / 2), cuuint64_t(H), cuuint64_t(B) };
     cuuint64_t strides[4] = { cuuint64_t(C) * 2, cuuint64_t(C) * 4, cuuint64_t(W) * C * 2, cuuint64_t(H) * W * C * 2 };
-    cuuint32_t box[5]     = { 16, 1, cuuint32_t(entries), cuuint32_t(rows), 1 };
+    cuuint32_t box[5]     = { 16, 1, cuuint32_t(entries), cuuint32_t(rows), cuuint32_t(images) };
     cuuint32_t es[5]      = { 1, 1, 1, 1, 1 };
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<uint16_t*>(base), dims, strides, box, es,
         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -922,16 +924,17 @@ cudaError_t mapPairs(CUtensorMap* m, const uint16_t* base, int B, int H, int W, 
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Plain view of a half-resolution NHWC BF16 tensor: (C, W0, H0, B), box 16 x entries, 32-byte
-// swizzle.
-cudaError_t mapRows(CUtensorMap* m, const uint16_t* base, int B, int H0, int W0, int C, int entries = kHaloEntries)
+// Plain view of a half-resolution NHWC BF16 tensor: (C, W0, H0, B), box 16 x entries x
+// images, 32-byte swizzle.
+cudaError_t mapRows(CUtensorMap* m, const uint16_t* base, int B, int H0, int W0, int C, int entries,
+    int images = 1)
 {
     auto enc = encodeTiled();
     if (!enc)
         return cudaErrorNotSupported;
     cuuint64_t dims[4]    = { cuuint64_t(C), cuuint64_t(W0), cuuint64_t(H0), cuuint64_t(B) };
     cuuint64_t strides[3] = { cuuint64_t(C) * 2, cuuint64_t(W0) * C * 2, cuuint64_t(H0) * W0 * C * 2 };
-    cuuint32_t box[4]     = { 16, cuuint32_t(entries), 1, 1 };
+    cuuint32_t box[4]     = { 16, cuuint32_t(entries), 1, cuuint32_t(images) };
     cuuint32_t es[4]      = { 1, 1, 1, 1 };
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<uint16_t*>(base), dims, strides, box, es,
         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1018,11 +1021,18 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     a.G         = (c.C0 + c.C1) / 16;
     a.G0        = c.C0 / 16;
     a.tilesX    = (c.W / 2 + 127) / 128;
+    // Images of at most 63 pairs a row share a tile's 128 MMA rows, each with its halo of two entries (rows
+    // that start on a halo entry are computed and dropped): four of 16 pairs are 70 rows of one tile where they
+    // were 16 of each of four.  With half the tiles to run, the rule below takes two rows a tile in place of
+    // four: 256 to 256 channels at 4 x 32 x 32 33 -> 22 us, the training step on four 256x256 crops 1364 -> 1228.
+    a.pitch  = std::min(c.W / 2 + 2, kHaloEntries);
+    a.images = a.tilesX > 1 ? 1 : std::min(c.B, (128 - c.W / 2) / a.pitch + 1);
+    const int groups = (c.B + a.images - 1) / a.images;
     int dev     = 0;
     if (cudaError_t ed = cudaGetDevice(&dev); ed != cudaSuccess)
         return ed;
     const int sms    = smCountOf(dev);
-    auto tilesOf     = [&](int rows) { return long(c.B) * ((c.H + rows - 1) / rows) * a.tilesX * a.nTiles; };
+    auto tilesOf     = [&](int rows) { return long(groups) * ((c.H + rows - 1) / rows) * a.tilesX * a.nTiles; };
     a.R              = tileRows(a.N);
     // Four rows of 64 channels take the whole TMEM, so a tile's epilogue holds up the next tile's MMAs in part;
     // but halo rows, weights and MMA operands are read for twice the outputs (414 cycles of MMAs for a 16-channel
@@ -1045,12 +1055,13 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     if (e0 != cudaSuccess)
         return e0;
     CUtensorMap m0, m1;
-    cudaError_t e = c.up0 ? mapRows(&m0, c.in0, c.B, c.H / 2, c.W / 2, c.C0) : mapPairs(&m0, c.in0, c.B, c.H, c.W, c.C0);
+    cudaError_t e = c.up0 ? mapRows(&m0, c.in0, c.B, c.H / 2, c.W / 2, c.C0, a.pitch, a.images)
+                           : mapPairs(&m0, c.in0, c.B, c.H, c.W, c.C0, a.pitch, 1, a.images);
     if (e != cudaSuccess)
         return e;
     if (c.C1 > 0)
     {
-        if ((e = mapPairs(&m1, c.in1, c.B, c.H, c.W, c.C1)) != cudaSuccess)
+        if ((e = mapPairs(&m1, c.in1, c.B, c.H, c.W, c.C1, a.pitch, 1, a.images)) != cudaSuccess)
             return e;
     }
     else
