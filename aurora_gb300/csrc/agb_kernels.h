@@ -199,16 +199,25 @@ struct ConvLaunch
 cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st);
 cudaError_t launchPackConvWeights(const float* w, int Cin, int Cout, int flip, uint16_t* out, cudaStream_t st);
 // Packs several layers' weights in one launch, each both ways (forward into out, data-gradient
-// into outFlip; either may be null).
+// into outFlip; either may be null).  With an Adam step (step.g not null) the layers' weights, and the Cout
+// biases behind each layer's weights, are updated first: g, m and v hold what belongs to params[k] at k.
 struct PackJob
 {
-    const float* w;
+    float* w;
     uint16_t* out;
     uint16_t* outFlip;
     int cin, cout;
 };
 constexpr int kMaxPackJobs = 16;
-cudaError_t launchPackConvWeightsMany(const PackJob* jobs, int count, cudaStream_t st);
+struct AdamStep
+{
+    const float* params;
+    const float* g;
+    float* m;
+    float* v;
+    float lr, b1, b2, eps, c1, c2; // c1, c2 = 1 - b^step
+};
+cudaError_t launchPackConvWeightsMany(const PackJob* jobs, int count, const AdamStep& step, cudaStream_t st);
 // dW[tap][ci][co] += sum over pixels of X[p + d][ci] dY[p][co] (X as c.in0 / c.in1 / c.up0; c.Cout
 // the layer's output channels: up to 128, or a multiple of 64 / 128 beyond; W even).
 cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, int smCount, cudaStream_t st);
@@ -254,7 +263,7 @@ public:
 
 private:
     cudaError_t alloc(void** p, size_t bytes, std::vector<void*>& list);
-    cudaError_t repack();
+    cudaError_t repack(const AdamStep& step);
     cudaError_t ensureShape(int B, int H, int W, bool training);
     static size_t pixels(int B, int H, int W, int level);
     ConvLaunch layerLaunch(int i, const uint16_t* x) const;

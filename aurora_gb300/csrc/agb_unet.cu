@@ -148,20 +148,6 @@ __global__ void __launch_bounds__(256) k_l1_loss(const float4* out32, const uint
     }
 }
 
-__global__ void k_adam(float* w, const float* g, float* m, float* v, long n, float lr, float b1, float b2,
-    float eps, float c1, float c2)
-{
-    for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x)
-    {
-        float gi = g[i];
-        float mi = b1 * m[i] + (1.f - b1) * gi;
-        float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i]     = mi;
-        v[i]     = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-}
-
 __device__ __forceinline__ float2 octEncode(float3 n)
 {
     float s = fabsf(n.x) + fabsf(n.y) + fabsf(n.z);
@@ -353,16 +339,16 @@ cudaError_t UnetDenoiser::init(uint64_t seed, cudaStream_t st, int smCount)
     if ((e = cudaMemcpyAsync(params_, h.data(), nParams_ * 4, cudaMemcpyHostToDevice, stream_)) != cudaSuccess)
         return e;
     step_ = 0;
-    return repack();
+    return repack(AdamStep{});
 }
 
-cudaError_t UnetDenoiser::repack()
+cudaError_t UnetDenoiser::repack(const AdamStep& step)
 {
-    // Every layer packed both ways (forward and data-gradient layouts) in one launch.
+    // Every layer, after the update if there is one, packed both ways (forward and data-gradient layouts) in one launch.
     PackJob jobs[kLayers];
     for (int i = 0; i < kLayers; i++)
         jobs[i] = PackJob{ params_ + wOff_[i], pack_ + packOff_[i], packFlip_ + packOff_[i], layerCin(i), layerCout(i) };
-    return launchPackConvWeightsMany(jobs, kLayers, stream_);
+    return launchPackConvWeightsMany(jobs, kLayers, step, stream_);
 }
 
 cudaError_t UnetDenoiser::ensureShape(int B, int H, int W, bool training)
@@ -626,12 +612,7 @@ cudaError_t UnetDenoiser::adam(float lr)
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     float c1 = 1.f - float(std::pow(double(b1), double(step_)));
     float c2 = 1.f - float(std::pow(double(b2), double(step_)));
-    k_adam<<<gridFor(long(nParams_)), 256, 0, stream_>>>(params_, grads_, adamM_, adamV_, long(nParams_), lr, b1, b2,
-        eps, c1, c2);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess)
-        return e;
-    return repack();
+    return repack(AdamStep{ params_, grads_, adamM_, adamV_, lr, b1, b2, eps, c1, c2 });
 }
 
 cudaError_t UnetDenoiser::setParams(const float* host)
@@ -639,7 +620,7 @@ cudaError_t UnetDenoiser::setParams(const float* host)
     cudaError_t e = cudaMemcpyAsync(params_, host, nParams_ * 4, cudaMemcpyHostToDevice, stream_);
     if (e != cudaSuccess)
         return e;
-    return repack();
+    return repack(AdamStep{});
 }
 
 double UnetDenoiser::flopsPerPixel(bool training)
