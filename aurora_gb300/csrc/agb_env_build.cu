@@ -559,8 +559,9 @@ __global__ void k_ref_index(const float* prob, uint32_t n, const uint32_t* tileS
 // subtracts, compares and notes where a large ended and what it was left with, and the block finds each
 // small's large from those notes.  w never grows within a large (deficits are >= 0), so the walk tests
 // groups of four smalls, or of sixteen while w is far from its end, with one comparison and goes back into
-// a group only when the large ends inside it.  Positions in [S, lrg) are larges already exhausted, whose probability is final and which follow
-// the smalls as smalls; a window beyond S ends at the lrg it started with.
+// a group only when the large ends inside it.  Positions in [S, lrg) are larges already exhausted,
+// whose probability is final and which follow the smalls as smalls; a window beyond S ends at the lrg it started
+// with.
 //
 // 512 x 256 texels of log-normal(0, 2) radiance with four suns: 16.4 ms with one warp that fetched,
 // compared and stored small by small, 2.5 ms with groups of four and a note per small, 0.75 ms so.

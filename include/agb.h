@@ -481,8 +481,8 @@ AGB_API agb_status agb_environment_alias(agb_context* ctx, agb_alias_entry* host
     uint64_t capacity, double* shading_integral, double* fp64_integral);
 
 /* Layout of the table agb_environment_set builds.  AGB_ENV_TABLE_REFERENCE (default) reproduces
- * the reference's AliasMap::build bit for bit (FP32 sequential integral and sweep; the sweep runs
- * on one warp).  The reference's environment MIS reuses one random pair for the table bucket and
+ * the reference's AliasMap::build bit for bit (FP32 sequential integral and sweep; one
+ * thread walks the sweep's chain).  The reference's environment MIS reuses one random pair for the table bucket and
  * for the BSDF lobe choice (ShadeFunctions.slang:146,220,237), so its converged image depends on
  * the bucket layout, and matching its images needs its layout.  AGB_ENV_TABLE_FP64 builds the
  * table from FP64 prefix sums (exact texel distribution, FP64 integral). */
