@@ -31,8 +31,11 @@ inline int traceCarveoutPercent()
 // 0.93 at 128; sampling kernel 1.55, 1.64, 1.33 and 1.65; MIS kernel 1.14, 1.08, 0.91 and 1.13 (512x512x16
 // of the small scene type).  Large blocks keep the warps that share an instruction cache near one another
 // in the code: the sampling kernel at 64 registers 1.33 ms with 128 threads per block, 1.22 with 512.
+// The surface kernel without the distant lights needs 118 registers and runs best at 80 (three blocks): 512x512x16
+// of the small scene type 6.18 ms at two blocks, 6.04 at three, 6.17 at four; 1920x1080x16 of the large one 46.7,
+// 46.0 and 46.2.
 constexpr int kShadeBlock     = 256; // surface kernel
-constexpr int kShadeMinBlocks = 2;
+constexpr int kShadeMinBlocks = 3;
 constexpr int kBsdfBlock      = 512; // sampling and MIS kernels
 constexpr int kBsdfMinBlocks  = 2;
 
