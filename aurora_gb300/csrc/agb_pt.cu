@@ -608,6 +608,19 @@ AGB_D float bounceClamp(const agb_frame_data& f)
     return f.indirect_bounce_clamp_scale > 0.f ? f.max_luminance * f.indirect_bounce_clamp_scale : 0.f;
 }
 
+// A shading warp's first queue entry.  A queue of at most one group of four warps per SM (a sixteenth of what the
+// launch takes in one turn) is dealt out in such groups, so that it does not fill a few SMs and leave the rest
+// idle: a lone 160x120 preview 650 -> 610 us, a lone 640x360 one-sample render of the large scene type 1.56 ->
+// 1.52 ms.  Beside other streams' kernels idle SMs are worth less than warps that share instructions: with queues
+// of up to a whole turn dealt out, that render takes 767 us beside two others instead of 743.
+constexpr uint32_t kShadeGroup = 128;
+AGB_D uint32_t firstOfWarp(uint32_t n)
+{
+    return n <= gridDim.x * blockDim.x / 16
+        ? (blockIdx.x + gridDim.x * (threadIdx.x / kShadeGroup)) * kShadeGroup + (threadIdx.x % kShadeGroup & ~31u)
+        : blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+}
+
 // kGraphs: the variant for scenes whose materials have node-graph programs (single-scene waves).
 template <bool kBatch, bool kGraphs = false>
 __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade(DevScene s, agb_frame_data f,
@@ -617,9 +630,9 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade(DevScene
     uint32_t stride = gridDim.x * blockDim.x;
     // Warp-uniform loop: every lane of a warp runs the same number of iterations so the queue
     // appends at the end of the body are executed by the whole warp.
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride)
+    for (uint32_t base = firstOfWarp(n); base < n; base += stride)
     {
-        uint32_t i     = base + threadIdx.x;
+        uint32_t i     = base + (threadIdx.x & 31);
         bool valid     = i < n;
         // A camera ray the ground plane turned into a reflection ray has nothing to shade here.
         if (valid && !depthLimit && s.ground.enabled && wb.hitInst[i] == kGroundAbsorbed)
@@ -826,9 +839,9 @@ __global__ void __launch_bounds__(kBsdfBlock, kBsdfMinBlocks) k_shade_scatter(De
 {
     uint32_t n      = wb.counters[bounce * kCounterStride + CNT_SCATTER];
     uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride)
+    for (uint32_t base = firstOfWarp(n); base < n; base += stride)
     {
-        uint32_t j     = base + threadIdx.x;
+        uint32_t j     = base + (threadIdx.x & 31);
         bool valid     = j < n;
         bool pushNext  = false;
         uint32_t p     = 0;
@@ -926,9 +939,9 @@ __global__ void __launch_bounds__(kBsdfBlock, kBsdfMinBlocks) k_shade_mis(DevSce
 {
     uint32_t n      = wb.counters[bounce * kCounterStride + CNT_SCATTER];
     uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride)
+    for (uint32_t base = firstOfWarp(n); base < n; base += stride)
     {
-        uint32_t j     = base + threadIdx.x;
+        uint32_t j     = base + (threadIdx.x & 31);
         bool valid     = j < n;
         uint32_t slots = 0;
         uint32_t p     = 0;
