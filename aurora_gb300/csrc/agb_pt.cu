@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade(DevScene
                         v3 emission = m.emissionColor * m.emission() * lerp3(splat(1.f), m.coatColor(), m.coat());
                         v3 so = dot(V, fr.N) < 0.f ? sh.geomPosition : sh.position;
                         contrib *= m.opacity / (1.f - P);
-                        // Hand the shading point to k_shade_scatter (environment MIS, the next
+                        // Hand the shading point to k_shade_scatter (distant lights, environment MIS, the next
                         // ray, Russian roulette), which runs with only those paths in its warps.
                         wb.pendEmission[p] = make_float4(emission.x, emission.y, emission.z, 0.f);
                         wb.shOrg[p]        = make_float4(so.x, so.y, so.z, 0.f);
@@ -811,7 +811,8 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade(DevScene
 // The hit shading after k_shade, in two kernels over the compacted shading points, each holding
 // one of the large Standard Surface entry points (the shading kernels' speed follows their
 // instruction-cache footprint):
-//   k_shade_scatter  draws the environment-MIS random pair and samples the BSDF with it
+//   k_shade_scatter  samples and evaluates the distant lights (ShadeFunctions.slang:51-89), draws the
+//                    environment-MIS random pair and samples the BSDF with it
 //                    (ShadeFunctions.slang:146-163), samples the indirect ray and applies Russian
 //                    roulette (ShadeFunctions.slang:263-310, HitShaderEntryPoints.slang:362-486),
 //                    appends the next ray and hands the MIS sample to k_shade_mis;
@@ -819,7 +820,7 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks) k_shade(DevScene
 //                    environment lookup, environment sample, evaluateMaterialAndPDF with the same
 //                    random pair), sets the pending-record bits and appends the resolve entry and
 //                    the shadow rays.
-// The random numbers are drawn in the reference's order (MIS pair, indirect pair, roulette); the
+// The random numbers are drawn in the reference's order (lights, MIS pair, indirect pair, roulette); the
 // MIS evaluation consumes none, so running it after the indirect sampling changes no value.
 
 // MIS sample handed from k_shade_scatter to k_shade_mis: kMisWords float4 per shading point,
