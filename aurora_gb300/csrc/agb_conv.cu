@@ -1093,28 +1093,37 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     if (c.Cout % a.N || (a.N != 16 && a.N != 32 && a.N != 48 && a.N != 64 && a.N != 96 && a.N != 128))
         return cudaErrorInvalidValue;
     a.coTiles  = c.Cout / a.N;
-    a.unitsX = (c.W / 2 + 63) / 64;
-    // Narrow images: a unit is as many rows as make 64 pairs (one row of an upsampled source, whose staged
-    // rows repeat).  Single rows leave up to three quarters of a unit's loads and MMAs to padding: the six
-    // weight gradients of 64x64 and 32x32 images in a training step on four 256x256 crops 350 us with
-    // them, 307 so (launches overlap), the step 1386 and 1364 us.
-    a.steps     = std::min(4, (c.W / 2 + 15) / 16);
-    a.rows      = c.up0 ? 1 : 4 / a.steps;
-    a.rowBlocks = (c.H + a.rows - 1) / a.rows;
-    a.entriesA  = 16 * a.steps + 2;
-    a.numUnits  = c.B * a.rowBlocks * a.unitsX;
+    a.unitsX   = (c.W / 2 + 63) / 64;
+    a.steps              = std::min(4, (c.W / 2 + 15) / 16);
     const int fixedItems = (a.T == 3 ? 1 : 3) * a.ciTiles * a.coTiles;
     const int sms        = smCount > 0 ? smCount : 148;
+    const bool twoSets   = 6 * a.N <= 512;
+    // Narrow images: a unit is as many rows as make 64 pairs, and its steps end with its rows (whole units of one row
+    // left up to three quarters of the loads and MMAs to padding).  A kernel with one set of accumulators sums
+    // no more rows in an item than two items per SM of single rows would, so that its sums are no longer for it:
+    // longer ones raised the error against 64 bits (256 to 256 channels at 4 x 32 x 32 1.7e-7 to 2.3e-7,
+    // so 1.6e-7).  An upsampled source, whose staged rows repeat, goes row by row.  Training step on four 256x256
+    // crops 1251 us with single rows in that kernel, 1232 so.
+    const int rowSplits = std::max(1, std::min(c.B * c.H, (2 * sms + fixedItems - 1) / fixedItems));
+    const int rowsEach  = (c.B * c.H + rowSplits - 1) / rowSplits;
+    a.rows              = c.up0 ? 1 : std::min(4 / a.steps, twoSets ? 4 : rowsEach);
+    a.rowBlocks         = (c.H + a.rows - 1) / a.rows;
+    a.entriesA          = 16 * a.steps + 2;
+    a.numUnits          = c.B * a.rowBlocks * a.unitsX;
     // A CTA takes a whole SM.  Two items per SM; where the kernel sums two halves of an item apart, two at most
     // (306 items on 152 SMs take three rounds), or one, if the item is short and its halves no longer than
     // a sum of the two-item split: every item pays a prologue, a pipeline fill and its reductions into dW
     // (64 to 64 channels at 4 x 128 x 128, 11 units an item: 20 us against 26), which long items hide.
     // One sum over a whole item would double the error against 64 bits.
-    const bool twoSets = 6 * a.N <= 512;
     auto splitsFor     = [&](int items) { return std::max(1, std::min(a.numUnits, items / fixedItems)); };
     auto perItem       = [&](int splits) { return (a.numUnits + splits - 1) / splits; };
     const int one = splitsFor(sms), two = splitsFor(2 * sms + fixedItems - 1);
-    if (!twoSets)
+    if (!twoSets && a.rows > 1)
+    {
+        const int each = rowsEach / a.rows;
+        a.splits       = (a.numUnits + each - 1) / each;
+    }
+    else if (!twoSets)
         a.splits = two;
     else
         a.splits = (perItem(one) + 1) / 2 <= perItem(two) && perItem(one) <= 32 ? one : splitsFor(2 * sms);
