@@ -570,16 +570,21 @@ AGB_API agb_status agb_context_memory(agb_context* ctx, uint64_t* bytes)
 {
     if (!ctx || !bytes)
         return fail(AGB_ERR_INVALID_ARG, "agb_context_memory: null argument");
-    uint64_t b = ctx->meshTable.bytes + ctx->imageTable.bytes + ctx->materials.bytes +
-        ctx->matTex.bytes + ctx->instances.bytes + ctx->tlasNodes.bytes + ctx->tlasOrder.bytes + ctx->traceInst.bytes +
-        ctx->layers.bytes + ctx->alias.bytes + ctx->pathState.bytes + ctx->queues.bytes +
-        ctx->counters.bytes + ctx->accMean.bytes + ctx->accSum.bytes + ctx->accComp.bytes +
-        ctx->lastSample.bytes + ctx->accMoments.bytes + ctx->post32.bytes + ctx->post8.bytes + ctx->aovDepth.bytes + ctx->aovNormal.bytes +
-        ctx->aovAlbedo.bytes + ctx->aovMotion.bytes + ctx->taaHistory[0].bytes + ctx->taaHistory[1].bytes +
-        uint64_t(ctx->envScratch.capacity) * 44 + ctx->stats.bytes;
+    // A part of another buffer counts with its owner, which keeps its allocation when the parts get smaller.
+    auto owned = [](std::initializer_list<const DevBuf*> bufs) {
+        uint64_t n = 0;
+        for (const DevBuf* d : bufs)
+            n += d->part ? 0 : d->bytes;
+        return n;
+    };
+    uint64_t b = owned({ &ctx->meshTable, &ctx->imageTable, &ctx->materials, &ctx->matTex, &ctx->instances,
+                     &ctx->tlasNodes, &ctx->tlasOrder, &ctx->traceInst, &ctx->layers, &ctx->alias, &ctx->pathState,
+                     &ctx->queues, &ctx->counters, &ctx->accArrays, &ctx->accMean, &ctx->accSum, &ctx->accComp,
+                     &ctx->lastSample, &ctx->accMoments, &ctx->post32, &ctx->post8, &ctx->aovDepth, &ctx->aovNormal,
+                     &ctx->aovAlbedo, &ctx->aovMotion, &ctx->taaHistory[0], &ctx->taaHistory[1], &ctx->stats }) +
+        uint64_t(ctx->envScratch.capacity) * 44;
     for (auto& g : ctx->geometries)
-        b += g->positions.bytes + g->normals.bytes + g->texcoords.bytes + g->verts.bytes + g->indices.bytes +
-            g->tris.bytes + g->nodes.bytes;
+        b += owned({ &g->arrays, &g->positions, &g->normals, &g->texcoords, &g->verts, &g->indices, &g->tris, &g->nodes });
     for (auto& i : ctx->images)
         b += i->data.bytes;
     for (auto& l : ctx->layerUVs)
