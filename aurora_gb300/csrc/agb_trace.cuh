@@ -245,7 +245,7 @@ constexpr int kNodeSteps = 2;
 // A Writer whose kRestart is true is called as write(scene, ray, hit?, hit, tmin) and returns
 // false to trace the same ray again from the tmin it sets (transparent shadows walk the hits
 // along the ray this way); endsAt(scene, instance) says that a hit on the instance ends the ray wherever
-// it lies, so the search stops there.  Other writers are called as write(ray, hit?, hit) and end the ray.
+// it lies, so the search stops there, with that instance as the hit's.  Other writers are called as write(ray, hit?, hit) and end the ray.
 template <class W, class = void>
 struct WriterRestarts
 {
@@ -442,7 +442,12 @@ AGB_D void persistentTrace(const DevScene& s, uint32_t n, uint32_t lanes, uint32
                 }
                 bool ends = kAnyHit;
                 if constexpr (WriterRestarts<Writer>::value)
+                {
                     ends = write.endsAt(s, inst);
+                    // It is the hit that counts, also where a surface in the same place was found first.
+                    if (ends)
+                        hit.inst = inst;
+                }
                 if (ends)
                 {
                     ref = kDone, sp = 0;
