@@ -634,14 +634,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3x3_tma(const __grid_consta
 // dW[tap][ci][co] += sum over pixels p of X[p + d(tap)][ci] dY[p][co], X = concat(up?(in0), in1):
 // a tcgen05 GEMM with M = input channels, N = output channels and K = pixels, both operands
 // MN-major (NHWC keeps a pixel's channels contiguous).  A unit of K is 128 output pixels of one
-// row (64 pairs), split by parity as in the forward pass: dY is staged as its even and odd rows
-// (64 entries each), X as the even and odd halo rows of 66 entries, so that the horizontal taps
-// are K offsets of 0, 1 or 2 entries into the same staged rows (an upsampled source is staged at
-// half resolution, the same row in both slots).  The vertical taps: when 3 x Cin <= 128 the M
-// rows are (dy, ci) - the three halo rows' channel groups are stacked at a uniform stride, so one
-// MMA covers all nine taps' rows for its horizontal tap - otherwise a work item takes one dy and
-// 128 input channels.  Accumulators: the three horizontal taps x N columns in TMEM, summed over
-// the item's units, then added to dW with vector reductions (red.global.add.v4.f32).
+// row (64 pairs), or up to four rows of a narrow image, split by parity as in the forward pass: dY is
+// staged as its even and odd entries (64 each), X as even and odd halo rows with two entries more a
+// row, so that the horizontal taps are K offsets of 0, 1 or 2 entries into the same staged rows (an
+// upsampled source is staged at half resolution, the same row in both slots).  The vertical taps: when
+// 3 x Cin <= 128 the M rows are (dy, ci) - the three halo rows' channel groups are stacked at a uniform
+// stride, so one MMA covers all nine taps' rows for its horizontal tap - otherwise a work item takes one
+// dy and 128 input channels.  Accumulators: the three horizontal taps x N columns in TMEM, one set of
+// them or (N <= 80) two, one for each half of the item's rows; their sums go through shared memory and
+// are added to dW by bulk reductions of whole rows of N floats.
 constexpr uint32_t kWgSlotA    = 2304; // 72 entries of 32 bytes: 1 x 66, 2 x 34 or 4 x 18 (64 pairs, offsets 0..2)
 constexpr uint32_t kWgSlotB    = 2048; // 64 entries
 constexpr int kWgThreads       = 192;  // producer, MMA issuer, 4 epilogue warps
@@ -667,12 +668,14 @@ struct WgradTmaArgs
 template <int N>
 constexpr uint32_t kWgRowBytes = uint32_t(N) * 4u + 16u;
 
-template <int N>
+// kHalves: the halves of an item may meet inside a unit (of several rows).  A variant of its own: the selects cost the
+// other units' issue of short MMAs 1.2 us of 28 (32 to 32 channels at 4 x 256 x 256).
+template <int N, bool kHalves>
 __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_constant__ CUtensorMap tm0,
     const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tmDy, const WgradTmaArgs a)
 {
-    // Where the TMEM holds two sets of the accumulators, an item sums the halves of its range apart and adds
-    // them at the end: the tensor core's FP32 accumulation loses a little with every unit, so a sum is
+    // Where the TMEM holds two sets of the accumulators, an item sums the halves of its rows apart and adds
+    // them at the end: the tensor core's FP32 accumulation loses a little with every step, so a sum is
     // kept no longer than half of what one item per SM has to cover.
     constexpr bool kTwoSets = 6 * N <= 512;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -692,7 +695,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
     const int dyIt = item / a.ciTiles; // the item's dy when T == 1
     const int u0   = sp * a.unitsPerItem;
     const int u1   = min(a.numUnits, u0 + a.unitsPerItem);
-    const int mid  = kTwoSets ? u0 + (u1 - u0 + 1) / 2 : u1; // units from here on go to the second set
+    // Image rows of a unit (its other rows lie below the image); rows (or whole units) of the item, and how many of
+    // them, the first half, go to the first set.
+    auto rowsIn         = [&](int u) { return min(a.rows, a.H - (u / a.unitsX) % a.rowBlocks * a.rows); };
+    const int itemRows  = !kHalves ? u1 - u0 : u1 - u0 == 1 ? rowsIn(u0) : (u1 - u0) * a.rows;
+    const int firstRows = kTwoSets ? (itemRows + 1) / 2 : itemRows;
 
     if (warp == 1)
         tc::tmemAlloc(&tmemBase, 512);
@@ -789,14 +796,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
             for (int k = 0; k < 4; k++)
                 stepA[k] = uint32_t((k / a.steps) * a.entriesA + (k % a.steps) * 16) * 2u;
             uint32_t it = 0;
+            bool second = false;
             for (int u = u0; u < u1; u++, it++)
             {
                 // Steps within the image: pairs and rows beyond it are staged as zeros.
                 const int pairs  = a.W / 2 - (u % a.unitsX) * 64;
                 const int across = min(a.steps, (pairs + 15) / 16);
-                const int steps  = across * min(a.rows, a.H - (u / a.unitsX) % a.rowBlocks * a.rows);
-                const bool first   = u == u0 || u == mid;
-                const uint32_t acc = tmem + (u < mid ? 0u : 3u * N);
+                const int steps  = across * rowsIn(u);
+                // Steps from `turn` on go to the second set.
+                const int turn = kHalves ? max(0, firstRows - (u - u0) * a.rows) * a.steps
+                    : u - u0 < firstRows ? 4 : 0;
                 const int s       = int(it % uint32_t(S));
                 const uint32_t ph = (it / uint32_t(S)) & 1u;
                 if (!tc::mbarWait(&full[s], ph))
@@ -811,21 +820,44 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
                 // atoms 256 bytes apart (stride byte offset).
                 const uint64_t aDesc0 = tc::smemDesc(aAddr, kWgSlotA, 256) | (uint64_t(6) << 61);
                 const uint64_t bDesc0 = tc::smemDesc(bAddr, kWgSlotB, 256) | (uint64_t(6) << 61);
-#pragma unroll
-                for (int par = 0; par < 2; par++)
-#pragma unroll
-                    for (int dx = 0; dx < 3; dx++)
+                // A pair of parities and a horizontal tap: the staged entries that they read.
+                auto shiftOf = [](int par, int dx) { return par == 0 ? (dx == 0 ? 0u : 1u) : (dx == 2 ? 2u : 1u); };
+                auto oddOf   = [](int par, int dx) { return par == 0 ? (dx == 1 ? 0u : 1u) : (dx == 1 ? 1u : 0u); };
+                if (kHalves && turn > 0 && turn < steps)
+                {
+                    // The halves meet inside the unit.
+#pragma unroll 1
+                    for (int i = 0; i < 6 * steps; i++)
                     {
-                        const uint32_t shift = par == 0 ? (dx == 0 ? 0u : 1u) : (dx == 2 ? 2u : 1u);
-                        const uint32_t odd   = par == 0 ? (dx == 1 ? 0u : 1u) : (dx == 1 ? 1u : 0u);
-                        const uint64_t ad    = aDesc0 + ((odd * 8u * kWgSlotA + shift * 32u) >> 4);
-                        const uint64_t bd    = bDesc0 + ((uint32_t(par) * (N / 16) * kWgSlotB) >> 4);
-#pragma unroll
-                        for (int ks = 0; ks < 4; ks++)
-                            if (ks < steps)
-                                tc::mma(acc + uint32_t(dx * N), ad + stepA[ks], bd + ((uint32_t(ks) * 16u * 32u) >> 4),
-                                    idesc, (first && par == 0 && ks == 0) ? 0u : 1u);
+                        const int ks = i % steps, dx = i / steps % 3, par = i / steps / 3;
+                        tc::mma(tmem + uint32_t(dx * N) + (ks < turn ? 0u : 3u * N),
+                            aDesc0 + ((oddOf(par, dx) * 8u * kWgSlotA + shiftOf(par, dx) * 32u) >> 4) +
+                                uint32_t((ks / a.steps) * a.entriesA + (ks % a.steps) * 16) * 2u,
+                            bDesc0 + ((uint32_t(par) * (N / 16) * kWgSlotB) >> 4) + uint32_t(ks * 32), idesc,
+                            par == 0 && (ks == turn || (u == u0 && ks == 0)) ? 0u : 1u);
                     }
+                    second = true;
+                }
+                else
+                {
+                    const uint32_t acc = tmem + (turn == 0 ? 3u * N : 0u);
+                    const bool first   = turn == 0 ? !second : u == u0;
+                    second             = turn == 0;
+#pragma unroll
+                    for (int par = 0; par < 2; par++)
+#pragma unroll
+                        for (int dx = 0; dx < 3; dx++)
+                        {
+                            const uint64_t ad = aDesc0 + ((oddOf(par, dx) * 8u * kWgSlotA + shiftOf(par, dx) * 32u) >> 4);
+                            const uint64_t bd = bDesc0 + ((uint32_t(par) * (N / 16) * kWgSlotB) >> 4);
+#pragma unroll
+                            for (int ks = 0; ks < 4; ks++)
+                                if (ks < steps)
+                                    tc::mma(acc + uint32_t(dx * N), ad + stepA[ks],
+                                        bd + ((uint32_t(ks) * 16u * 32u) >> 4), idesc,
+                                        (first && par == 0 && ks == 0) ? 0u : 1u);
+                        }
+                }
                 tc::commit(&empty[s]);
             }
             tc::commit(&accFull);
@@ -861,10 +893,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_tma(const __grid_c
                     uint32_t v[16], v2[16];
                     const uint32_t col = tmem + (uint32_t(quad * 32) << 16) + uint32_t(dx * N + c0);
                     tc::tmemLoad16(col, v);
-                    if (mid < u1)
+                    if (firstRows < itemRows)
                         tc::tmemLoad16(col + 3u * N, v2);
                     tc::tmemWaitLoad();
-                    if (mid < u1)
+                    if (firstRows < itemRows)
 #pragma unroll
                         for (int q = 0; q < 16; q++)
                             v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(v2[q]));
@@ -1099,34 +1131,48 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     const int sms        = smCount > 0 ? smCount : 148;
     const bool twoSets   = 6 * a.N <= 512;
     // Narrow images: a unit is as many rows as make 64 pairs, and its steps end with its rows (whole units of one row
-    // left up to three quarters of the loads and MMAs to padding).  A kernel with one set of accumulators sums
-    // no more rows in an item than two items per SM of single rows would, so that its sums are no longer for it:
-    // longer ones raised the error against 64 bits (256 to 256 channels at 4 x 32 x 32 1.7e-7 to 2.3e-7,
-    // so 1.6e-7).  An upsampled source, whose staged rows repeat, goes row by row.  Training step on four 256x256
-    // crops 1251 us with single rows in that kernel, 1232 so.
-    const int rowSplits = std::max(1, std::min(c.B * c.H, (2 * sms + fixedItems - 1) / fixedItems));
-    const int rowsEach  = (c.B * c.H + rowSplits - 1) / rowSplits;
-    a.rows              = c.up0 ? 1 : std::min(4 / a.steps, twoSets ? 4 : rowsEach);
-    a.rowBlocks         = (c.H + a.rows - 1) / a.rows;
-    a.entriesA          = 16 * a.steps + 2;
-    a.numUnits          = c.B * a.rowBlocks * a.unitsX;
+    // left up to three quarters of the loads and MMAs to padding).  No sum takes more rows than two items per SM
+    // of single rows would: the tensor core's FP32 accumulation loses a little with every step.  Longer sums
+    // raised the error against 64 bits: 256 to 256 channels at 4 x 32 x 32, one set of accumulators, 1.7e-7 to
+    // 2.3e-7; 64 to 64 channels at 1 x 32 x 32, two sets, 1.12e-7 to 1.28e-7 (0.91e-7 so).  An upsampled source, whose staged
+    // rows repeat, goes row by row.  Training step on four 256x256 crops 1251 us with single rows where one set is
+    // kept, 1232 so.
+    const int lines    = c.B * c.H * a.unitsX; // units of one row
+    const int twoItems = std::max(1, std::min(lines, (2 * sms + fixedItems - 1) / fixedItems));
+    const int each     = (lines + twoItems - 1) / twoItems; // rows of the longest sum
+    a.entriesA         = 16 * a.steps + 2;
+    auto setRows       = [&](int rows) {
+        a.rows      = rows;
+        a.rowBlocks = (c.H + rows - 1) / rows;
+        a.numUnits  = c.B * a.rowBlocks * a.unitsX;
+    };
     // A CTA takes a whole SM.  Two items per SM; where the kernel sums two halves of an item apart, two at most
-    // (306 items on 152 SMs take three rounds), or one, if the item is short and its halves no longer than
-    // a sum of the two-item split: every item pays a prologue, a pipeline fill and its reductions into dW
-    // (64 to 64 channels at 4 x 128 x 128, 11 units an item: 20 us against 26), which long items hide.
-    // One sum over a whole item would double the error against 64 bits.
-    auto splitsFor     = [&](int items) { return std::max(1, std::min(a.numUnits, items / fixedItems)); };
-    auto perItem       = [&](int splits) { return (a.numUnits + splits - 1) / splits; };
-    const int one = splitsFor(sms), two = splitsFor(2 * sms + fixedItems - 1);
-    if (!twoSets && a.rows > 1)
+    // (306 items on 152 SMs take three rounds), or one, if the item is short and its halves are no longer than
+    // that: every item pays a prologue, a pipeline fill and its reductions into dW (64 to 64 channels at
+    // 4 x 128 x 128, 11 units an item: 20 us against 26), which long items hide.  One sum over a whole
+    // item would double the error against 64 bits.
+    auto splitsFor = [&](int items) { return std::max(1, std::min(a.numUnits, items / fixedItems)); };
+    auto dealt     = [&](int n) { return (a.numUnits + n - 1) / n; }; // the units dealt out in n parts, or in parts of n
+    auto onePerSm  = [&]() {
+        const int units = dealt(splitsFor(sms));
+        return (units * a.rows + 1) / 2 <= each && units <= 32;
+    };
+    const int maxRows = c.up0 ? 1 : std::min(4 / a.steps, twoSets ? 2 * each : each);
+    setRows(maxRows);
+    if (twoSets)
     {
-        const int each = rowsEach / a.rows;
-        a.splits       = (a.numUnits + each - 1) / each;
+        while (!onePerSm() && a.rows > 1)
+            setRows(a.rows - 1);
+        if (onePerSm())
+            a.splits = splitsFor(sms);
+        else
+        {
+            setRows(maxRows);
+            a.splits = std::max(splitsFor(2 * sms), dealt(2 * each / a.rows));
+        }
     }
-    else if (!twoSets)
-        a.splits = two;
     else
-        a.splits = (perItem(one) + 1) / 2 <= perItem(two) && perItem(one) <= 32 ? one : splitsFor(2 * sms);
+        a.splits = dealt(each / a.rows);
     a.unitsPerItem = (a.numUnits + a.splits - 1) / a.splits;
     a.splits       = (a.numUnits + a.unitsPerItem - 1) / a.unitsPerItem;
     a.numItems     = fixedItems * a.splits;
@@ -1153,8 +1199,13 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     // The stages, or the epilogue's rows (three times 128) in their place.
     const size_t smem = std::max<size_t>(std::max<size_t>(size_t(a.stages) * a.stageBytes, 120 * 1024),
         size_t(3) * 128 * (size_t(a.N) * 4 + 16));
-    auto kern = a.N == 128 ? k_conv_wgrad_tma<128> : a.N == 96 ? k_conv_wgrad_tma<96> : a.N == 64 ? k_conv_wgrad_tma<64>
-        : a.N == 48 ? k_conv_wgrad_tma<48> : a.N == 32 ? k_conv_wgrad_tma<32> : k_conv_wgrad_tma<16>;
+    const bool halves = twoSets && a.rows > 1;
+    auto kern = a.N == 128 ? k_conv_wgrad_tma<128, false>
+        : a.N == 96        ? k_conv_wgrad_tma<96, false>
+        : a.N == 64        ? (halves ? k_conv_wgrad_tma<64, true> : k_conv_wgrad_tma<64, false>)
+        : a.N == 48        ? (halves ? k_conv_wgrad_tma<48, true> : k_conv_wgrad_tma<48, false>)
+        : a.N == 32        ? (halves ? k_conv_wgrad_tma<32, true> : k_conv_wgrad_tma<32, false>)
+                           : (halves ? k_conv_wgrad_tma<16, true> : k_conv_wgrad_tma<16, false>);
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) != cudaSuccess)
         return e;
     return launchOverlapped(kern, unsigned(a.numItems), kWgThreads, smem, st, m0, m1, md, a);
