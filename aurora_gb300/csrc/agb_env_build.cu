@@ -324,16 +324,21 @@ __global__ void k_ref_lum(const float4* rgba, uint32_t width, uint32_t n, const 
 // every thread the sum that the sequential loop would reach before its addends; a chunk is taken as a
 // whole while no thread's sum leaves the binade.  The first thread that leaves it (or that holds an
 // addend that is negative or not finite) adds its own addends one by one, and the next chunk starts
-// behind them in the new binade.  A sum that is zero, subnormal, infinite or NaN is carried on one by
-// one, in runs that double while that lasts.
+// behind them in the new binade.  One thread adds one by one, from shared memory, in runs that double
+// while that lasts: while the sum is zero, subnormal, infinite or NaN, and after a chunk that such an
+// addend stopped early (a chunk takes as long as 1,300 addends of a run).
 //
-// Bound by the load and scan latency of one block, a few us per chunk of 8,192 addends and per binade:
-// 512 x 256 texels 0.63 ms by the sequential loop (10 cycles an addend), 0.11 ms so.  Whole-number
+// Bound by the load and scan latency of one block, 3 us per chunk of 8,192 addends and per binade:
+// 512 x 256 texels 0.63 ms by the sequential loop (10 cycles an addend), 0.11 ms so.  Where a run is what is left:
+// 2048 x 1024 texels of which half, or one in a hundred, are negative 7.7 and 7.6 ms (10.0 by the
+// sequential loop; 872 and 68 with every chunk tried), with an infinite one 5.7.  Whole-number
 // arithmetic: the same maps from FP64 products took 0.63 ms too (two FP64 lanes' worth per SM).
-constexpr int kSumThreads   = 1024;
-constexpr int kSumPer       = 8;
-constexpr uint32_t kSumFull = 1u << 24; // one past the binade's last integer
-constexpr uint32_t kSumCap  = 1u << 25; // saturation of the maps: any value beyond kSumFull does
+constexpr int kSumThreads    = 1024;
+constexpr int kSumPer        = 8;
+constexpr uint32_t kSumFull  = 1u << 24; // one past the binade's last integer
+constexpr uint32_t kSumCap   = 1u << 25; // saturation of the maps: any value beyond kSumFull does
+constexpr uint32_t kSumRun   = 8192;     // longest one-by-one run
+constexpr uint32_t kSumShort = 512;      // a chunk that an addend stops before this many is followed by such a run
 
 struct SumMap
 {
@@ -350,16 +355,18 @@ __device__ __forceinline__ SumMap composeSum(SumMap f, SumMap g)
 __global__ void __launch_bounds__(kSumThreads) k_ref_seq_sum(const float* v, uint32_t n, float* out)
 {
     __shared__ SumMap warpMap[kSumThreads / 32];
+    __shared__ float run[kSumRun];
     __shared__ float accS;
     __shared__ uint32_t posS;
     __shared__ int firstStop;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     float acc       = 0.f;
     uint32_t pos    = 0;
-    uint32_t serial = 64; // addends of the next one-by-one run
+    uint32_t serial = 64;    // addends of the next one-by-one run
+    bool oneByOne   = false; // the last chunk did not get far
     while (pos < n)
     {
-        if (!(acc >= 1.17549435e-38f && acc < __int_as_float(0x7f800000)))
+        if (oneByOne || !(acc >= 1.17549435e-38f && acc < __int_as_float(0x7f800000)))
         {
             if (acc == 0.f)
             {
@@ -383,21 +390,25 @@ __global__ void __launch_bounds__(kSumThreads) k_ref_seq_sum(const float* v, uin
                     continue;
             }
             const uint32_t cnt = min(serial, n - pos);
+            for (uint32_t k = t; k < cnt; k += kSumThreads)
+                run[k] = v[pos + k];
+            __syncthreads();
             if (t == 0)
             {
                 float s = acc;
+#pragma unroll 16
                 for (uint32_t k = 0; k < cnt; k++)
-                    s = __fadd_rn(s, v[pos + k]);
+                    s = __fadd_rn(s, run[k]);
                 accS = s;
             }
             __syncthreads();
             acc = accS;
             pos += cnt;
-            serial = min(serial * 2u, 8192u);
+            serial   = min(serial * 2u, kSumRun);
+            oneByOne = false;
             __syncthreads();
             continue;
         }
-        serial = 64;
         const int e        = int(__float_as_uint(acc) >> 23); // biased exponent, 1 .. 254
         const uint32_t m0  = (__float_as_uint(acc) & 0x7fffffu) | 0x800000u;
         const uint32_t at  = pos + uint32_t(t) * kSumPer;
@@ -488,11 +499,16 @@ __global__ void __launch_bounds__(kSumThreads) k_ref_seq_sum(const float* v, uin
                     if (at + k < n)
                         s = __fadd_rn(s, x[k]);
             accS = s;
-            posS = pos + uint32_t(stop == kSumThreads ? kSumThreads : stop + 1) * kSumPer;
+            // A multiple of 8; bit 0: the chunk stopped at an addend that the maps do not describe.
+            posS = pos + uint32_t(stop == kSumThreads ? kSumThreads : stop + 1) * kSumPer + (odd ? 1u : 0u);
         }
         __syncthreads();
-        acc = accS;
-        pos = posS;
+        acc               = accS;
+        const uint32_t to = posS;
+        const bool early  = to - pos < kSumShort;
+        oneByOne          = early && (to & 1u);
+        serial            = early ? serial : 64;
+        pos               = to & ~1u;
         __syncthreads();
     }
     if (t == 0)
