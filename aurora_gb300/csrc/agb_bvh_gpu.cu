@@ -761,6 +761,41 @@ __global__ void __launch_bounds__(kSubThreads) k_bvh_subtree(const float* boxes,
     }
 }
 
+// See readBvhTop: one warp, a level at a time.
+__global__ void __launch_bounds__(32) k_bvh_top(const BNode* nodes, int32_t root, BNode* out)
+{
+    __shared__ int32_t at[kBvhTopNodes];
+    static_assert(kBvhTopNodes < 32, "a lane per node");
+    const int t = threadIdx.x;
+    if (t < kBvhTopNodes)
+        at[t] = t == 0 ? root : -1;
+    __syncwarp();
+    for (int level = 0; level < kBvhTopLevels; level++)
+    {
+        if (t < (1 << level))
+        {
+            const int k = (1 << level) - 1 + t;
+            BNode n{};
+            if (at[k] >= 0)
+            {
+                n = nodes[at[k]];
+                if (level + 1 < kBvhTopLevels && n.ref.x >= 0)
+                {
+                    at[2 * k + 1] = n.ref.x;
+                    n.ref.x       = 2 * k + 1;
+                }
+                if (level + 1 < kBvhTopLevels && n.ref.y >= 0)
+                {
+                    at[2 * k + 2] = n.ref.y;
+                    n.ref.y       = 2 * k + 2;
+                }
+            }
+            out[k] = n;
+        }
+        __syncwarp();
+    }
+}
+
 __global__ void k_tri_boxes(const float* positions, const uint32_t* indices, uint32_t ntri, float* boxes)
 {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntri; t += gridDim.x * blockDim.x)
@@ -954,6 +989,17 @@ cudaError_t buildTlasGpu(const float* boxesHost, uint32_t count, int maxDepth, G
         cudaSuccess)
         return e;
     return cudaMemcpyAsync(orderOut, s.order, size_t(count) * 4, cudaMemcpyDeviceToDevice, st);
+}
+
+cudaError_t readBvhTop(GpuBvhScratch& s, const BNode* nodes, int32_t root, BNode* host, cudaStream_t st)
+{
+    // The large nodes' arrays, at least two records twice, are free once the tree is built.
+    static_assert(sizeof(BigNode) * 4 >= sizeof(BNode) * kBvhTopNodes, "room for the top of the tree");
+    BNode* top = static_cast<BNode*>(s.big);
+    k_bvh_top<<<1, 32, 0, st>>>(nodes, root, top);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(host, top, sizeof(BNode) * kBvhTopNodes, cudaMemcpyDeviceToHost, st);
 }
 
 void freeGpuBvhScratch(GpuBvhScratch& s)

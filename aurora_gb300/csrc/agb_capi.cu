@@ -364,12 +364,10 @@ agb_status ensureAccum(agb_context* ctx, uint32_t W, uint32_t H)
     return AGB_OK;
 }
 
-// Collects the child boxes of the BLAS down to kCoverDepth levels (or to a leaf, or to a node that
-// is not among the `avail` nodes at hand) into out; a mesh whose root is a leaf keeps its bounds.
-// BLAS node order in memory.  The GPU builder numbers nodes level by level.  AGB_BLAS_LAYOUT=dfs
-// lays them out depth first with a node's two interior children side by side (a path's nodes
-// close together, both children of a node in one or two cache lines): the children of node n are
-// placed together, and the pairs of child 0's subtree follow before child 1's.  The tree (and so
+// BLAS node order in memory.  The GPU builder numbers the large nodes level by level, then each subtree of at most
+// 512 triangles in one run.  AGB_BLAS_LAYOUT=dfs lays them out depth first with a node's two interior
+// children side by side (a path's nodes close together, both children of a node in one or two cache
+// lines): the children of node n are placed together, and the pairs of child 0's subtree follow before child 1's.  The tree (and so
 // every hit) is the same.  Measured on the large configuration: closest-hit 138.2 -> 137.8 ms,
 // shadow 97.8 -> 97.5 ms per frame, for a host round trip of the nodes per build, so the builder's
 // order stays the default.
@@ -411,9 +409,10 @@ void layoutDepthFirst(const std::vector<BNode>& in, int32_t root, std::vector<BN
     }
 }
 
+// Collects the child boxes of the BLAS down to kBvhTopLevels levels (or to a leaf) into out; a mesh whose root
+// is a leaf keeps its bounds.  nodes: `avail` of them, with the tree's top levels among them.
 void coverBoxes(const BNode* nodes, uint32_t avail, int32_t root, const float* bounds, std::vector<float>& out)
 {
-    const int kCoverDepth = 5;
     out.clear();
     if (root < 0 || uint32_t(root) >= avail)
     {
@@ -436,7 +435,7 @@ void coverBoxes(const BNode* nodes, uint32_t avail, int32_t root, const float* b
             int32_t ref     = side == 0 ? n.ref.x : n.ref.y;
             const float4 xy = side == 0 ? n.c0xy : n.c1xy;
             float z0 = side == 0 ? n.cz.x : n.cz.z, z1 = side == 0 ? n.cz.y : n.cz.w;
-            if (ref >= 0 && uint32_t(ref) < avail && it.depth + 1 < kCoverDepth)
+            if (ref >= 0 && uint32_t(ref) < avail && it.depth + 1 < kBvhTopLevels)
                 stack.push_back({ ref, it.depth + 1 });
             else
             {
@@ -699,15 +698,14 @@ AGB_API agb_status agb_geometry_create(agb_context* ctx, const float* positions,
             "agb_geometry_create: GPU BVH build");
         if (depth > kBlasMaxDepth)
             return fail(AGB_ERR_LIMIT, "agb_geometry_create: BLAS deeper than the traversal stack allows");
-        // The builder numbers the large nodes first, level by level, then each small subtree's in one run:
-        // the first ones are the top of the tree (all of a mesh whose top five levels hold subtrees).
-        std::vector<BNode> top(std::min<uint32_t>(nodeCount, 4096));
-        if (!top.empty())
-            AGB_CUDA(cudaMemcpyAsync(top.data(), s.nodes, top.size() * sizeof(BNode), cudaMemcpyDeviceToHost,
-                         ctx->stream),
-                "read BVH top");
+        std::vector<BNode> top;
+        if (root >= 0)
+        {
+            top.resize(kBvhTopNodes);
+            AGB_CUDA(readBvhTop(s, s.nodes, root, top.data(), ctx->stream), "read BVH top");
+        }
         AGB_CUDA(cudaStreamSynchronize(ctx->stream), "upload geometry");
-        coverBoxes(top.data(), uint32_t(top.size()), root, g->bounds, g->cover);
+        coverBoxes(top.data(), uint32_t(top.size()), root >= 0 ? 0 : root, g->bounds, g->cover);
         if (nodeCount && blasLayoutDepthFirst())
         {
             // Depth-first order with each node's interior children side by side (see layoutDepthFirst).

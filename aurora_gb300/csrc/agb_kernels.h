@@ -337,6 +337,12 @@ cudaError_t buildBlasGpu(const float* positions, const uint32_t* indices, uint32
 cudaError_t buildTlasGpu(const float* boxesHost, uint32_t count, int maxDepth, GpuBvhScratch& s, BNode* nodes,
     uint32_t nodeCapacity, int32_t* orderOut, int32_t* rootOut, int32_t* depthOut, uint32_t* nodeCountOut,
     cudaStream_t st);
+// The top levels of a tree just built (root a node, not a leaf) as a binary heap: node k's children that are nodes
+// among those levels are at 2 k + 1 and 2 k + 2, and its refs say so.  Queues the copy to host memory
+// (kBvhTopNodes entries, the slots of no node zero) on the stream.
+constexpr int kBvhTopLevels = 5;
+constexpr int kBvhTopNodes  = (1 << kBvhTopLevels) - 1;
+cudaError_t readBvhTop(GpuBvhScratch& s, const BNode* nodes, int32_t root, BNode* host, cudaStream_t st);
 void freeGpuBvhScratch(GpuBvhScratch& s);
 
 // agb_unit.cu
