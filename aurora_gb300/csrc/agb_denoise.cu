@@ -145,7 +145,10 @@ cudaError_t takeTcError(int* flag, cudaStream_t st)
         e = cudaStreamSynchronize(st);
     if (e != cudaSuccess || *flag == 0)
         return e;
-    return cudaMemset(dev, 0, sizeof(int));
+    // On the same stream: the default stream may be busy, and the next call on st would see the old flag or lose
+    // one that is set meanwhile.
+    e = cudaMemsetAsync(dev, 0, sizeof(int), st);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(st);
 }
 
 cudaError_t tcErrorFlag(int** flag) { return cudaGetSymbolAddress(reinterpret_cast<void**>(flag), g_tcError); }
