@@ -731,8 +731,10 @@ AGB_API agb_status agb_server_memory(agb_server* srv, uint64_t* scene_bytes, uin
  *     env_filter_linear are ignored) and the frame data set on it.  Views must not repeat, must
  *     agree on is_force_opaque_shadows_enabled, and their scenes must have no ground plane.
  *     Asynchronous: the views' own streams wait for the batch, so agb_accum_read and the denoiser
- *     calls on a view see its result; agb_batch_poll reports completion.  With stats it waits and
- *     fills them (paths, rays, launches, device time). */
+ *     calls on a view see its result; agb_batch_poll reports completion.  With stats it waits after
+ *     every wave and fills them (paths, rays, launches, device time); the images are the same.  Such
+ *     a call launches every stage by itself, which its launch count shows; without stats a bounce's
+ *     shadow rays and the next bounce's closest-hit rays share a launch, which is the faster way. */
 typedef struct agb_batch agb_batch;
 AGB_API agb_status agb_batch_create(int32_t device, void* cuda_stream, uint64_t max_paths_in_flight,
     agb_batch** out);
