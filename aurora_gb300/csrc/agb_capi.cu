@@ -367,10 +367,10 @@ agb_status ensureAccum(agb_context* ctx, uint32_t W, uint32_t H)
 // BLAS node order in memory.  The GPU builder numbers the large nodes level by level, then each subtree of at most
 // 512 triangles in one run.  AGB_BLAS_LAYOUT=dfs lays them out depth first with a node's two interior
 // children side by side (a path's nodes close together, both children of a node in one or two cache
-// lines): the children of node n are placed together, and the pairs of child 0's subtree follow before child 1's.  The tree (and so
-// every hit) is the same.  Measured on the large configuration: closest-hit 138.2 -> 137.8 ms,
-// shadow 97.8 -> 97.5 ms per frame, for a host round trip of the nodes per build, so the builder's
-// order stays the default.
+// lines): the children of node n are placed together, and the pairs of child 0's subtree follow before
+// child 1's.  The tree (and so every hit) is the same.  Measured on the large configuration: closest-hit
+// 138.2 -> 137.8 ms, shadow 97.8 -> 97.5 ms per frame, for a host round trip of the nodes per build, so
+// the builder's order stays the default.
 bool blasLayoutDepthFirst()
 {
     const char* v = getenv("AGB_BLAS_LAYOUT");

@@ -1055,8 +1055,8 @@ cudaError_t launchConv3x3(const ConvLaunch& c, cudaStream_t st)
     a.tilesX    = (c.W / 2 + 127) / 128;
     // Images of at most 63 pairs a row share a tile's 128 MMA rows, each with its halo of two entries (rows
     // that start on a halo entry are computed and dropped): four of 16 pairs are 70 rows of one tile where they
-    // were 16 of each of four.  With half the tiles to run, the rule below takes two rows a tile in place of
-    // four: 256 to 256 channels at 4 x 32 x 32 33 -> 22 us, the training step on four 256x256 crops 1364 -> 1228.
+    // would be 16 of each of four.  256 to 256 channels at 4 x 32 x 32 are 64 tiles of two rows so, 22 us, and with a
+    // tile an image (by the rule below) 128 of four rows, 33 us; the training step on four 256x256 crops 1228 and 1364.
     a.pitch  = std::min(c.W / 2 + 2, kHaloEntries);
     a.images = a.tilesX > 1 ? 1 : std::min(c.B, (128 - c.W / 2) / a.pitch + 1);
     const int groups = (c.B + a.images - 1) / a.images;
@@ -1134,9 +1134,9 @@ cudaError_t launchConvWgrad(const ConvLaunch& c, const uint16_t* dy, float* dw, 
     // left up to three quarters of the loads and MMAs to padding).  No sum takes more rows than two items per SM
     // of single rows would: the tensor core's FP32 accumulation loses a little with every step.  Longer sums
     // raised the error against 64 bits: 256 to 256 channels at 4 x 32 x 32, one set of accumulators, 1.7e-7 to
-    // 2.3e-7; 64 to 64 channels at 1 x 32 x 32, two sets, 1.12e-7 to 1.28e-7 (0.91e-7 so).  An upsampled source, whose staged
-    // rows repeat, goes row by row.  Training step on four 256x256 crops 1251 us with single rows where one set is
-    // kept, 1232 so.
+    // 2.3e-7; 64 to 64 channels at 1 x 32 x 32, two sets, 1.12e-7 to 1.28e-7 (0.91e-7 so).  An upsampled source,
+    // whose staged rows repeat, goes row by row.  Training step on four 256x256 crops 1251 us with single rows
+    // where one set is kept, 1232 so.
     const int lines    = c.B * c.H * a.unitsX; // units of one row
     const int twoItems = std::max(1, std::min(lines, (2 * sms + fixedItems - 1) / fixedItems));
     const int each     = (lines + twoItems - 1) / twoItems; // rows of the longest sum

@@ -245,7 +245,8 @@ constexpr int kNodeSteps = 2;
 // A Writer whose kRestart is true is called as write(scene, ray, hit?, hit, tmin) and returns
 // false to trace the same ray again from the tmin it sets (transparent shadows walk the hits
 // along the ray this way); endsAt(scene, instance) says that a hit on the instance ends the ray wherever
-// it lies, so the search stops there, with that instance as the hit's.  Other writers are called as write(ray, hit?, hit) and end the ray.
+// it lies, so the search stops there, with that instance as the hit's.  Other writers are called as
+// write(ray, hit?, hit) and end the ray.
 template <class W, class = void>
 struct WriterRestarts
 {
